@@ -388,6 +388,21 @@ int xs_tri_levels(int n, const int *rowptr, const int *colidx, int upper, int *l
 int xs_tri_tiles(int n, const int *rowptr, const int *colidx, int upper, int tx, int ty, int tz, int *info, int *perm,
                  int *prp, int *pci, int *tile_pos, int *tile_lvl, int *lvl_ptr, int *halo_ptr, int *halo_row);
 
+/* Line schedule of a strict triangle's exact solve (host-only; see
+ * xs_set_trsv_lines).  Step x + al*Y + be*Z (Y = y + c*z, Z = z in the
+ * triangle's logical coordinates) is solved for all lines of a patch of
+ * ty*tz lines at once.  info[24] = {fits, nx, ny, nz, c, al, be, lines per
+ * patch, ty, tz, reach in Y and Z, ring columns per row of lines, ring
+ * columns, patch grid in Y and Z, patches, steps per patch, diagonals,
+ * exported lines, halo lines, longest step distance}; when fits is 0 nothing
+ * else is written.  Optional outputs (NULL to skip; at most 32 diagonals, 128
+ * lines and 64 halo lines): per diagonal delta (steps back), shift (ring
+ * columns back) and offq (logical row offset), patch[2*patches] (Y, Z in
+ * ticket order), rank_of[patch grid], halo[2*halo lines] (Y, Z relative to
+ * the patch), exp_of[lines per patch]. */
+int xs_tri_lines(int n, const int *rowptr, const int *colidx, int upper, int *info, int *delta, int *shift, int *offq,
+                 int *patch, int *rank_of, int *halo, int *exp_of);
+
 /* LU solve that allocates nothing (no counterpart in the reference).
  * z = (L D U')^{-1} x with the factors in the seqilu0 layout (L strict lower
  * CSR with unit diagonal implied, dinv = 1/u_ii, U' = dinv-row-scaled strict
@@ -450,6 +465,14 @@ int xs_set_persistent_iteration(int enable);
  * XS_TRSV_TILE_MIN_ROWS set it at first use.  Fixed when a preconditioner is
  * built: set before factorising. */
 int xs_set_trsv_tiles(int enable, int tx, int ty, int tz, int min_rows);
+/* Line-scheduled exact triangular solves: mode 1 (default) uses them instead
+ * of boxes, level order or the single-CTA solve for triangles of at least
+ * min_rows rows (default 512) whose entries lie on at most 32 diagonals of a
+ * grid with little padding (stencil ILU(0), ParILUT fill of a stencil),
+ * unless xs_set_trsv_tiles turned grid schedules off or set a box size;
+ * 2 also with a box size set; 0 never.  Results are bitwise the same.
+ * Fixed when a preconditioner is built. */
+int xs_set_trsv_lines(int mode, int min_rows);
 /* Exact LU solves of systems with at most max_rows rows, whose solution
  * vector fits in one SM's shared memory (FP64: 25600 rows), run in one CTA
  * that walks the dependency levels with a block barrier between them

@@ -1,0 +1,187 @@
+"""Line-scheduled exact triangular solves on the GPU.
+
+The schedule (xs_tri_lines) replaces the row-per-thread dependency flags of
+the reference's sync-free solves (hip/Precond/gpuparilu.cpp:257-364) on
+stencil patterns.  It changes only which thread computes a row, when, and
+where a dependency is read from; each row's entries are summed in the same
+order with the same operations, so FP64 results are bitwise the oracle's
+LUsolve (hip/HostMatrix/HostMatrixCSR.cpp:385-409) and reduced precisions
+bitwise the level-ordered solve's."""
+import numpy as np
+import pytest
+
+import oracle
+from test_lines import P5, P7, P9, P27, _stencil
+from xsolver_b200 import stencils as st
+
+pytestmark = pytest.mark.gpu
+
+
+class lines_mode:
+    """Line schedule forced for every qualifying triangle (mode 2) or off (0)."""
+
+    def __init__(self, mode):
+        self.mode = mode
+
+    def __enter__(self):
+        from xsolver_b200 import _lib
+
+        assert _lib.lib().xs_set_trsv_lines(self.mode, 8) == 0
+
+    def __exit__(self, *exc):
+        from xsolver_b200 import _lib
+
+        _lib.lib().xs_set_trsv_lines(1, 512)
+
+
+def _dev(a, cuda):
+    import torch
+
+    return torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+
+
+def _lusolve(P, x, cuda, reps=1, t=False):
+    import torch
+
+    dx = _dev(x, cuda)
+    out = []
+    for _ in range(reps):
+        z = torch.full_like(dx, float("nan"))
+        (P.lusolve_t if t else P.lusolve)(dx, z)
+        P.sync()
+        out.append(z.cpu().numpy())
+    return out
+
+
+# one line and one step around a patch (32-128 lines) and a stage (8 steps),
+# several patches in Y and Z, lines shorter and longer than the ring (64)
+SHAPES = [((9, 11, 10), P7), ((17, 33, 9), P7), ((16, 8, 64), P7), ((33, 17, 71), P7), ((40, 41, 42), P7),
+          ((12, 13, 14), P27), ((17, 33, 20), P27), ((129, 63), P5), ((128, 128), P5), ((7, 300), P5), ((300, 9), P9),
+          ((11, 12, 13), [o for o in P27 if sum(map(abs, o)) <= 2])]
+
+
+@pytest.mark.parametrize("shape,offs", SHAPES)
+def test_lusolve_fp64_bitwise_vs_oracle(cuda, shape, offs):
+    from xsolver_b200.api import Plan
+
+    A = _stencil(shape, offs)
+    F = oracle.ilu0(A)
+    x = st.rhs_uniform(A.n, 7)
+    with lines_mode(2):
+        P = Plan(A).factor("ilu0")
+        for z in _lusolve(P, x, cuda, reps=4):  # both halves of the exchange buffer, re-armed
+            assert np.array_equal(z, oracle.lusolve(F, x))
+        (zt,) = _lusolve(P, x, cuda, t=True)
+        assert np.allclose(zt, oracle.lusolve_t(F, x), rtol=1e-12, atol=1e-12)
+
+
+def test_parilut_fill_bitwise_vs_oracle(cuda):
+    from xsolver_b200.api import Plan
+
+    A = st.convdiff3d_27pt(24)
+    F = oracle.parilut(A, fill=2.0, sweeps=5, droptol=1e-4)
+    x = st.rhs_uniform(A.n, 5)
+    with lines_mode(2):
+        P = Plan(A).factor("parilut", sweeps=5, fill=2.0, droptol=1e-4)
+        (z,) = _lusolve(P, x, cuda)
+    assert np.array_equal(z, oracle.lusolve(F, x))
+
+
+@pytest.mark.parametrize("prec", ["fp32", "bf16", "fp16"])
+@pytest.mark.parametrize("shape,offs", [((17, 33, 20), P27), ((33, 17, 71), P7), ((129, 63), P5)])
+def test_reduced_precision_equals_level_ordered(cuda, prec, shape, offs):
+    from xsolver_b200 import _lib
+    from xsolver_b200.api import Plan
+
+    A = _stencil(shape, offs)
+    x = st.rhs_uniform(A.n, 9).astype(np.float32)
+    outs = []
+    _lib.lib().xs_set_trsv_block_rows(0)
+    try:
+        for mode in (2, 0):
+            with lines_mode(mode):
+                P = Plan(A).factor("ilu0").set_factor_precision(prec)
+                outs.append(_lusolve(P, x, cuda, reps=2))
+    finally:
+        _lib.lib().xs_set_trsv_block_rows(1 << 30)
+    for z in outs[0]:
+        assert np.array_equal(z, outs[1][0])
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 8, 16])
+@pytest.mark.parametrize("shape,offs", [((33, 17, 30), P7), ((12, 13, 14), P27)])
+def test_several_right_hand_sides_equal_single_solves(cuda, k, shape, offs):
+    import torch
+    from xsolver_b200.api import Plan
+
+    A = _stencil(shape, offs)
+    F = oracle.ilu0(A)
+    X = np.stack([st.rhs_uniform(A.n, c) for c in range(k)], 1)
+    with lines_mode(2):
+        P = Plan(A).factor("ilu0")
+        dX = _dev(X, cuda)
+        for _ in range(2):
+            Z = torch.full_like(dX, float("nan"))
+            P.lusolve_batch(dX, Z)
+            P.sync()
+            for c in range(k):
+                assert np.array_equal(Z[:, c].cpu().numpy(), oracle.lusolve(F, X[:, c]))
+
+
+def test_one_triangle_on_lines_the_other_not(cuda):
+    """A lower triangle that qualifies beside an upper one that does not: each
+    kernel re-arms what the other polls, in either order."""
+    from xsolver_b200 import CSRMatrix, _lib
+    from xsolver_b200.api import Plan
+
+    A = _stencil((20, 21, 22), P7, 2)
+    rows = np.repeat(np.arange(A.n), np.diff(A.rowptr))
+    drop = np.random.default_rng(0).random(A.nnz) < 0.5
+    x = st.rhs_uniform(A.n, 3)
+    _lib.lib().xs_set_trsv_block_rows(0)
+    try:
+        for part in (A.colidx > rows, A.colidx < rows):
+            keep = ~(drop & part)
+            rp = np.zeros(A.n + 1, np.int64)
+            np.cumsum(np.bincount(rows[keep], minlength=A.n), out=rp[1:])
+            B = CSRMatrix(A.n, rp, A.colidx[keep], A.val[keep])
+            F = oracle.ilu0(B)
+            with lines_mode(2):
+                P = Plan(B).factor("ilu0")
+                for z in _lusolve(P, x, cuda, reps=3):
+                    assert np.array_equal(z, oracle.lusolve(F, x))
+    finally:
+        _lib.lib().xs_set_trsv_block_rows(1 << 30)
+
+
+def test_wait_times_out_and_recovers(cuda):
+    """A patch that waits for a value nothing publishes: the bounded wait gives
+    up after about 1 s, the error is reported, and the plan works again."""
+    from xsolver_b200.api import Plan, XsError
+
+    A = st.poisson3d_7pt(24)
+    F = oracle.ilu0(A)
+    x = st.rhs_uniform(A.n, 1)
+    with lines_mode(2):
+        P = Plan(A).factor("ilu0")
+        P.debug_break_dependency(A.n - 1, True)
+        with pytest.raises(XsError) as e:
+            _lusolve(P, x, cuda)
+        assert e.value.code == 5  # XS_ERR_TRSV_TIMEOUT
+        P.debug_break_dependency(A.n - 1, False)
+        for z in _lusolve(P, x, cuda, reps=2):
+            assert np.array_equal(z, oracle.lusolve(F, x))
+
+
+def test_infinities_and_nans_pass_through(cuda):
+    """Infinities and NaNs in the right-hand side spread as in the sequential
+    solve; a NaN that is not the marker is published like any value."""
+    from xsolver_b200.api import Plan
+
+    A = _stencil((17, 18, 19), P7)
+    F = oracle.ilu0(A)
+    x = st.rhs_uniform(A.n, 2)
+    x[1000], x[3000] = np.inf, np.nan
+    with lines_mode(2):
+        (z,) = _lusolve(Plan(A).factor("ilu0"), x, cuda)
+    assert np.array_equal(z, oracle.lusolve(F, x), equal_nan=True)

@@ -818,8 +818,7 @@ static void load_tri_values(Handle &h, TriDev &T, const double *vals, const Fact
     auto one = [&](auto &pbuf, auto &nbuf) {
         using FT = std::remove_pointer_t<decltype(pbuf.p)>;
         if (pos) {
-            if (pbuf.n != (size_t)m) pbuf.alloc(m, 8);  // padded: the box solve stages whole 4-byte words
-            if (T.nnz) k_gather_convert<FT><<<g, 256, 0, h.s>>>(T.nnz, T.src.p, vals, pbuf.p);
+            gather_pos_values<FT>(T, vals, pbuf, h.s);
         } else {
             pbuf.free();
         }
@@ -841,12 +840,12 @@ static void load_dinv(Handle &h, const double *vals, const long *diagsrc, bool n
 {
     const int g = geom().sms * 4;
     TriDev &U = h.M.U;
-    if (U.dinv64.n != (size_t)h.n) { U.dinv64.alloc(h.n, 4); U.dinv64_nat.alloc(h.n); }
-    k_gather_dinv<double><<<g, 256, 0, h.s>>>(h.n, U.perm.p, diagsrc, vals, U.dinv64.p);
+    if (U.dinv64_nat.n != (size_t)h.n) U.dinv64_nat.alloc(h.n);
+    gather_pos_dinv<double>(U, diagsrc, vals, U.dinv64, h.s);
     k_gather_dinv<double><<<g, 256, 0, h.s>>>(h.n, nullptr, diagsrc, vals, U.dinv64_nat.p);
     if (need32) {
-        if (U.dinv32.n != (size_t)h.n) { U.dinv32.alloc(h.n, 4); U.dinv32_nat.alloc(h.n); }
-        k_gather_dinv<float><<<g, 256, 0, h.s>>>(h.n, U.perm.p, diagsrc, vals, U.dinv32.p);
+        if (U.dinv32_nat.n != (size_t)h.n) U.dinv32_nat.alloc(h.n);
+        gather_pos_dinv<float>(U, diagsrc, vals, U.dinv32, h.s);
         k_gather_dinv<float><<<g, 256, 0, h.s>>>(h.n, nullptr, diagsrc, vals, U.dinv32_nat.p);
     }
     check_launch();
@@ -1539,16 +1538,14 @@ static void adjoint_prepare(Handle &h)
         const int g = geom().sms * 4;
         for (TriDev *D : {&T.L, &T.U}) {
             long m = std::max<long>(D->nnz, 1);
-            D->pv64.alloc(m, 8);
+            gather_pos_values<double>(*D, vals, D->pv64, h.s);
             D->nv64.alloc(m);
             if (D->nnz) {
-                k_gather_convert<double><<<g, 256, 0, h.s>>>(D->nnz, D->src.p, vals, D->pv64.p);
                 k_gather_convert<double><<<g, 256, 0, h.s>>>(D->nnz, D->src_nat.p, vals, D->nv64.p);
             }
         }
-        T.U.dinv64.alloc(n, 4);
         T.U.dinv64_nat.alloc(n);
-        k_gather_dinv<double><<<g, 256, 0, h.s>>>(n, T.U.perm.p, diagsrc, vals, T.U.dinv64.p);
+        gather_pos_dinv<double>(T.U, diagsrc, vals, T.U.dinv64, h.s);
         k_gather_dinv<double><<<g, 256, 0, h.s>>>(n, nullptr, diagsrc, vals, T.U.dinv64_nat.p);
         check_launch();
         T.ensure_buffers64(h.s);
@@ -1973,6 +1970,41 @@ int xs_tri_tiles(int n, const int *rp, const int *ci, int upper, int tx, int ty,
         };
         put(perm, P.perm); put(prp, P.prp); put(pci, P.pci); put(tile_pos, P.tile_pos);
         put(tile_lvl, P.tile_lvl); put(lvl_ptr, P.lvl_ptr); put(halo_ptr, P.halo_ptr); put(halo_row, P.halo_row);
+    });
+}
+
+int xs_tri_lines(int n, const int *rp, const int *ci, int upper, int *info, int *delta, int *shift, int *offq, int *patch,
+                 int *rank_of, int *halo, int *exp_of)
+{
+    return guarded([&] {
+        if (n < 0 || !rp || !info || (!ci && n > 0 && rp[n] > 0)) throw Status(XS_ERR_INVALID);
+        TileGrid G;
+        LineHost H;
+        std::memset(info, 0, sizeof(int) * 24);
+        if (!tile_detect(n, rp, ci, upper != 0, G) || !line_layout(n, rp[n], G, geom().sms, H)) return;
+        const LineGeo &g = H.g;
+        const int v[22] = {1,    g.nx, g.ny, g.nz,   g.c,   g.al,  g.be,     g.L,      g.ty, g.tz, g.ry,
+                           g.rz, g.py, g.npad, g.npy, g.npz, g.npatch, g.nsteps, g.D,  g.E,  g.nh, g.maxd};
+        std::memcpy(info, v, sizeof(v));
+        auto put = [](int *dst, const int *v, size_t m) {
+            if (dst && m) std::memcpy(dst, v, sizeof(int) * m);
+        };
+        put(delta, g.delta, g.D);
+        put(shift, g.shift, g.D);
+        put(offq, g.offq, g.D);
+        put(patch, H.patch.data(), H.patch.size());
+        put(rank_of, H.rank_of.data(), H.rank_of.size());
+        put(halo, H.halo.data(), H.halo.size());
+        put(exp_of, H.exp_of.data(), H.exp_of.size());
+    });
+}
+
+int xs_set_trsv_lines(int mode, int min_rows)
+{
+    return guarded([&] {
+        if (mode < 0 || mode > 2 || (mode && min_rows < 8)) throw Status(XS_ERR_INVALID);
+        tile_tuning().lines = mode;
+        if (mode) tile_tuning().line_min_rows = min_rows;
     });
 }
 

@@ -381,9 +381,12 @@ __global__ void __launch_bounds__(TILEM_THREADS) k_trsv_tiles_multi(TileArgs<dou
 struct BatchPrecond {
     DBuf<double> lb, ub;  // readiness buffers, n*k each (NaN sentinel)
     DBuf<unsigned> ticket;
+    LineXchg<double> lx, ux;  // line-scheduled triangles
     int n = 0, k = 0;
-    void ensure(int nn, int kk, cudaStream_t s)
+    void ensure(const PrecondDev &M, int nn, int kk, cudaStream_t s)
     {
+        if (M.L.lined) line_xchg_ensure(lx, M.L.lines.g, kk, s);
+        if (M.U.lined) line_xchg_ensure(ux, M.U.lines.g, kk, s);
         if (n == nn && k == kk && lb.p) return;
         n = nn;
         k = kk;
@@ -399,6 +402,8 @@ struct BatchPrecond {
         if (!lb.p) return;
         k_fill_sentinel<double><<<256, 256, 0, s>>>(lb.p, (int)((size_t)n * k));
         k_fill_sentinel<double><<<256, 256, 0, s>>>(ub.p, (int)((size_t)n * k));
+        line_xchg_rearm(lx, s);
+        line_xchg_rearm(ux, s);
         check_launch();
     }
 };
@@ -415,10 +420,17 @@ inline int tiles_multi_kc(const TriDev &T, int k)
 template <bool UPPER>
 inline void launch_trsv_multi(const TriDev &T, int k, unsigned *ticket, const double *dinv, const double *rhs,
                               double *self, double *out_user, double *reset_other, const int *all_done, int *err,
-                              cudaStream_t s)
+                              cudaStream_t s, LineXchg<double> &X)
 {
     const int bo = trsv_tuning().backoff_ns;
-    if (T.tiled) {
+    if (T.lined) {
+        double *out = out_user ? out_user : self;
+        const double *pv = T.pv64.p;
+        const int kc = line_kc(T.lines.g, k);
+        if (kc == 1) launch_trsv_lines<double, double, double, UPPER, 1>(T.lines, pv, dinv, X, k, rhs, out, reset_other, all_done, err, s);
+        else if (kc == 2) launch_trsv_lines<double, double, double, UPPER, 2>(T.lines, pv, dinv, X, k, rhs, out, reset_other, all_done, err, s);
+        else launch_trsv_lines<double, double, double, UPPER, 4>(T.lines, pv, dinv, X, k, rhs, out, reset_other, all_done, err, s);
+    } else if (T.tiled) {
         const int kc = tiles_multi_kc(T, k);
         const int ng = (k + kc - 1) / kc;
         const size_t smem = TileSmemM::of(T.t_max_rows, T.t_max_halo, T.t_max_entries, kc).total;
@@ -486,9 +498,10 @@ inline void batch_apply(PrecondDev &M, BatchPrecond &B, int k, const double *X, 
     } else if (M.type == PC_JACOBI) {
         k_bdiag_scale<<<geom().sms * 4, 256, 0, s>>>(m, k, M.jdiag64.p, X, Z, all_done);
     } else {
-        B.ensure(n, k, s);
-        launch_trsv_multi<false>(M.L, k, B.ticket.p, nullptr, X, B.lb.p, nullptr, B.ub.p, all_done, M.err, s);
-        launch_trsv_multi<true>(M.U, k, B.ticket.p, M.U.dinv64.p, B.lb.p, B.ub.p, Z, B.lb.p, all_done, M.err, s);
+        B.ensure(M, n, k, s);
+        double *arm_u = M.U.lined ? nullptr : B.ub.p, *arm_l = M.L.lined ? nullptr : B.lb.p;
+        launch_trsv_multi<false>(M.L, k, B.ticket.p, nullptr, X, B.lb.p, nullptr, arm_u, all_done, M.err, s, B.lx);
+        launch_trsv_multi<true>(M.U, k, B.ticket.p, M.U.dinv64.p, B.lb.p, B.ub.p, Z, arm_l, all_done, M.err, s, B.ux);
     }
     check_launch();
 }
@@ -548,7 +561,7 @@ struct BatchPcg {
         KState *st = S.st.p;
         int *ad = S.all_done.p;
         const RedSlot sl = S.slot();
-        if (M.type != PC_NONE && M.type != PC_JACOBI) BP.ensure(n, k, s);  // before any capture
+        if (M.type != PC_NONE && M.type != PC_JACOBI) BP.ensure(M, n, k, s);  // before any capture
         const int G = batch_grid(), TB = batch_block(k);
         k_bspmv<BS_RESID><<<G, TB, 0, s>>>(n, k, A.rp, A.ci, A.v, X, R, B, st, ad, sl);
         batch_apply(M, BP, k, R, Z, ad, s);

@@ -1054,19 +1054,19 @@ inline void ilut_to_tri(cudaStream_t s, int n, ParilutResult &R, TriDev &L, TriD
         }
         const long m = std::max<long>(T.nnz, 1);
         const int g = geom().sms * 4;
-        T.pv64.alloc(m, 8); T.nv64.alloc(m);
+        T.nv64.alloc(m);
+        gather_pos_values<double>(T, vals, T.pv64, s);
         if (T.nnz) {
-            k_gather_convert<double><<<g, 256, 0, s>>>(T.nnz, T.src.p, vals, T.pv64.p);
             k_gather_convert<double><<<g, 256, 0, s>>>(T.nnz, T.src_nat.p, vals, T.nv64.p);
         }
         if (need32) {
-            T.pv32.alloc(m, 8); T.nv32.alloc(m); T.pvbf.alloc(m, 8); T.nvbf.alloc(m); T.pvh.alloc(m, 8); T.nvh.alloc(m);
+            T.nv32.alloc(m); T.nvbf.alloc(m); T.nvh.alloc(m);
+            gather_pos_values<float>(T, vals, T.pv32, s);
+            gather_pos_values<__nv_bfloat16>(T, vals, T.pvbf, s);
+            gather_pos_values<__half>(T, vals, T.pvh, s);
             if (T.nnz) {
-                k_gather_convert<float><<<g, 256, 0, s>>>(T.nnz, T.src.p, vals, T.pv32.p);
                 k_gather_convert<float><<<g, 256, 0, s>>>(T.nnz, T.src_nat.p, vals, T.nv32.p);
-                k_gather_convert<__nv_bfloat16><<<g, 256, 0, s>>>(T.nnz, T.src.p, vals, T.pvbf.p);
                 k_gather_convert<__nv_bfloat16><<<g, 256, 0, s>>>(T.nnz, T.src_nat.p, vals, T.nvbf.p);
-                k_gather_convert<__half><<<g, 256, 0, s>>>(T.nnz, T.src.p, vals, T.pvh.p);
                 k_gather_convert<__half><<<g, 256, 0, s>>>(T.nnz, T.src_nat.p, vals, T.nvh.p);
             }
         }
@@ -1077,12 +1077,12 @@ inline void ilut_to_tri(cudaStream_t s, int n, ParilutResult &R, TriDev &L, TriD
     host_both([&] { up(L, R.hlrp, R.hlci, R.lrp.p, R.lci.p, false, R.lv.p); },
               [&] { up(U, R.hurp, R.huci, R.urp.p, R.uci.p, true, R.uv.p); });
     const int g = geom().sms * 4;
-    U.dinv64.alloc(n, 4); U.dinv64_nat.alloc(n);
-    k_gather_dinv<double><<<g, 256, 0, s>>>(n, U.perm.p, R.diag_ident.p, R.dinv.p, U.dinv64.p);
+    U.dinv64_nat.alloc(n);
+    gather_pos_dinv<double>(U, R.diag_ident.p, R.dinv.p, U.dinv64, s);
     k_gather_dinv<double><<<g, 256, 0, s>>>(n, nullptr, R.diag_ident.p, R.dinv.p, U.dinv64_nat.p);
     if (need32) {
-        U.dinv32.alloc(n, 4); U.dinv32_nat.alloc(n);
-        k_gather_dinv<float><<<g, 256, 0, s>>>(n, U.perm.p, R.diag_ident.p, R.dinv.p, U.dinv32.p);
+        U.dinv32_nat.alloc(n);
+        gather_pos_dinv<float>(U, R.diag_ident.p, R.dinv.p, U.dinv32, s);
         k_gather_dinv<float><<<g, 256, 0, s>>>(n, nullptr, R.diag_ident.p, R.dinv.p, U.dinv32_nat.p);
     }
     check_launch();

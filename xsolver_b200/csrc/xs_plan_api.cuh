@@ -261,6 +261,16 @@ int xs_plan_debug_break_dependency(xs_plan_t p, int position, int enable)
         TriDev &L = h.M.L;
         if (position < 0 || position >= L.n) throw Status(XS_ERR_INVALID);
         XS_CUDA(cudaStreamSynchronize(h.s));
+        if (L.lined) {
+            // line schedule: the patch that holds the row waits for a value
+            // that never comes, so the wait runs out
+            const LineGeo &g = L.lines.g;
+            const int z = position / (g.nx * g.ny), Y = position / g.nx % g.ny + g.c * z;
+            std::vector<int> rank((size_t)g.npy * g.npz);
+            XS_CUDA(cudaMemcpy(rank.data(), L.lines.rank_of.p, sizeof(int) * rank.size(), cudaMemcpyDeviceToHost));
+            L.lines.brk = enable ? rank[(size_t)(z / g.tz) * g.npy + Y / g.ty] : -1;
+            return;
+        }
         if (L.tiled) {
             // box layout: the box holding `position` waits for one of its own
             // rows as if it were a halo value; that row is published only

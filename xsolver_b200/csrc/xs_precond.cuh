@@ -41,6 +41,8 @@ struct PrecondDev {
     TriDev L, U;
     DBuf<double> lbuf64, ubuf64, tmp64a, tmp64b, tmp64c;
     DBuf<float> lbuf32, ubuf32, tmp32a, tmp32b, tmp32c;
+    LineXchg<double> lx64, ux64;  // exchange buffers of line-scheduled solves
+    LineXchg<float> lx32, ux32;
     int *err = nullptr;
     bool have_factors = false;
 
@@ -53,6 +55,8 @@ struct PrecondDev {
             k_fill_sentinel<double><<<256, 256, 0, s>>>(ubuf64, n);
             check_launch();
         }
+        if (L.lined) line_xchg_ensure(lx64, L.lines.g, 1, s);
+        if (U.lined) line_xchg_ensure(ux64, U.lines.g, 1, s);
     }
     void ensure_buffers32(cudaStream_t s)
     {
@@ -63,6 +67,8 @@ struct PrecondDev {
             k_fill_sentinel<float><<<256, 256, 0, s>>>(ubuf32, n);
             check_launch();
         }
+        if (L.lined) line_xchg_ensure(lx32, L.lines.g, 1, s);
+        if (U.lined) line_xchg_ensure(ux32, U.lines.g, 1, s);
     }
     // temporaries of the Jacobi-sweep mode
     void ensure_sweep_buffers(bool need32)
@@ -75,6 +81,10 @@ struct PrecondDev {
     {
         if (lbuf64.n) { k_fill_sentinel<double><<<256, 256, 0, s>>>(lbuf64, n); k_fill_sentinel<double><<<256, 256, 0, s>>>(ubuf64, n); }
         if (lbuf32.n) { k_fill_sentinel<float><<<256, 256, 0, s>>>(lbuf32, n); k_fill_sentinel<float><<<256, 256, 0, s>>>(ubuf32, n); }
+        line_xchg_rearm(lx64, s);
+        line_xchg_rearm(ux64, s);
+        line_xchg_rearm(lx32, s);
+        line_xchg_rearm(ux32, s);
         check_launch();
     }
 
@@ -143,10 +153,15 @@ struct PrecondDev {
         if constexpr (std::is_same<VT, double>::value) dinv = U.dinv64.p;
         else dinv = U.dinv32.p;
         VT *lb = lbuf<VT>(), *ub = ubuf<VT>();
+        // a line-scheduled triangle polls its exchange buffer, not lb / ub
+        VT *arm_u = U.lined ? nullptr : ub, *arm_l = L.lined ? nullptr : lb;
+        LineXchg<VT> *lx, *ux;
+        if constexpr (std::is_same<VT, double>::value) { lx = &lx64; ux = &ux64; }
+        else { lx = &lx32; ux = &ux32; }
         if (half == 0)
-            launch_trsv<VT, FT, DT, false>(L, (const DT *)nullptr, x, lb, (VT *)nullptr, ub, done_flag, err, s);
+            launch_trsv<VT, FT, DT, false>(L, (const DT *)nullptr, x, lb, (VT *)nullptr, arm_u, done_flag, err, s, *lx);
         else
-            launch_trsv<VT, FT, DT, true>(U, dinv, lb, ub, z, lb, done_flag, err, s);
+            launch_trsv<VT, FT, DT, true>(U, dinv, lb, ub, z, arm_l, done_flag, err, s, *ux);
     }
     // one half of the exact solve in the configured precision (timing)
     template <typename VT>

@@ -405,6 +405,12 @@ __global__ void k_fill_sentinel(VT *b, int n)
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b[i] = Sentinel<VT>::value();
 }
 
+}  // namespace xs
+
+#include "xs_trsv_lines.cuh"  // line-scheduled exact solves (uses msub, k_fill_sentinel)
+
+namespace xs {
+
 // ---------------------------------------------------------------- Jacobi-sweep mode
 // Reference GPU path (DeviceMatrixCSR.cpp:14-58, 281-304): y = 0, then k times
 // y = x - L_off y   (L) / y = dinv*x - U' y  (U, row-scaled form).
@@ -903,7 +909,15 @@ struct TriDev {
     int ntiles = 0, tile_elems = 0;  // tile_elems: shared-memory values per box (rows + halo)
     int t_max_rows = 0, t_max_halo = 0, t_max_entries = 0;
     DBuf<int> t_pos, t_lvl, t_lptr, t_hptr, t_hrow, lvperm;
-    const int *level_perm() const { return tiled ? lvperm.p : perm.p; }
+    // line schedule (xs_trsv_lines.cuh): pv*/dinv* of the exact solve then
+    // hold the schedule's slots, perm/prp/pci/src stay empty, lvperm keeps
+    // the level order as with boxes
+    bool lined = false;
+    LinePlan lines;
+    const int *level_perm() const { return tiled || lined ? lvperm.p : perm.p; }
+    // elements of a value copy in the order of the exact solve
+    size_t pos_elems() const { return lined ? (size_t)lines.g.slots() * lines.g.D : (size_t)std::max<long>(nnz, 1); }
+    size_t pos_rows() const { return lined ? (size_t)lines.g.slots() : (size_t)n; }
     template <typename FT>
     TileArgs<FT> targs() const
     {
@@ -971,6 +985,38 @@ __global__ void k_gather_dinv(int n, const int *__restrict__ perm, const long *_
         int r = perm ? perm[p] : p;
         dst[p] = (DT)vals[diagsrc[r]];
     }
+}
+
+// values (and, for U, the inverse diagonal) in the order of the exact solve
+template <typename FT>
+inline void gather_pos_values(const TriDev &T, const double *vals, DBuf<FT> &dst, cudaStream_t s)
+{
+    const int g = geom().sms * 4;
+    if (dst.n != T.pos_elems()) dst.alloc(T.pos_elems(), 8);  // padded: the box solve stages whole 4-byte words
+    if (T.nnz == 0) return;
+    if (T.lined) {
+        const LinePlan &P = T.lines;
+        const int gl = geom().sms * 8;
+        if (P.g.mask8()) {
+            auto kern = T.upper ? k_line_vals<true, uint8_t, FT> : k_line_vals<false, uint8_t, FT>;
+            kern<<<gl, 256, 0, s>>>(P.g, P.patch.p, P.mask8.p, T.rp_nat.p, T.src_nat.p, vals, dst.p);
+        } else {
+            auto kern = T.upper ? k_line_vals<true, uint32_t, FT> : k_line_vals<false, uint32_t, FT>;
+            kern<<<gl, 256, 0, s>>>(P.g, P.patch.p, P.mask32.p, T.rp_nat.p, T.src_nat.p, vals, dst.p);
+        }
+    } else {
+        k_gather_convert<FT><<<g, 256, 0, s>>>(T.nnz, T.src.p, vals, dst.p);
+    }
+    check_launch();
+}
+template <typename DT>
+inline void gather_pos_dinv(const TriDev &U, const long *diagsrc, const double *vals, DBuf<DT> &dst, cudaStream_t s)
+{
+    const int g = geom().sms * 4;
+    if (dst.n != U.pos_rows()) dst.alloc(U.pos_rows(), 4);
+    if (U.lined) k_line_dinv<DT><<<g, 256, 0, s>>>(U.lines.g, U.lines.patch.p, diagsrc, vals, dst.p);
+    else k_gather_dinv<DT><<<g, 256, 0, s>>>(U.n, U.perm.p, diagsrc, vals, dst.p);
+    check_launch();
 }
 
 }  // namespace xs
@@ -1063,15 +1109,45 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
     // boxes shrink until the rows and halo of one fit in shared memory
     TileHostPlan TP;
     T.tiled = false;
+    T.lined = false;
+    T.lines = LinePlan();
     T.t_pos.free(); T.t_lvl.free(); T.t_lptr.free(); T.t_hptr.free(); T.t_hrow.free(); T.lvperm.free();
-    if (!T.chunked && tile_tuning().enable && n >= tile_tuning().min_rows) {
-        Trace tr_tile("    box analysis", s);
+    const bool want_lines = !T.chunked && tile_tuning().enable && n >= tile_tuning().line_min_rows &&
+                            (tile_tuning().lines == 2 || (tile_tuning().lines && !tile_tuning().user_box));
+    const bool want_tiles = !T.chunked && tile_tuning().enable && n >= tile_tuning().min_rows;
+    if (want_lines || want_tiles) {
+        Trace tr_tile("    grid analysis", s);
         TileTuning tt = tile_tuning();
         TileGrid G;
+        LineHost H;
         Trace tr_det("      grid detection", s);
         const bool on_grid = tile_detect(n, rp.data(), ci.data(), upper, G);
         tr_det.stop();
-        if (on_grid) {
+        if (on_grid && want_lines && line_layout(n, T.nnz, G, geom().sms, H)) {
+            T.lined = true;
+            LinePlan &P = T.lines;
+            P.g = H.g;
+            auto up = [&](DBuf<int> &b, const std::vector<int> &v) {
+                b.alloc(std::max<size_t>(v.size(), 1));
+                if (!v.empty()) b.upload(v.data(), v.size(), s);
+            };
+            up(P.patch, H.patch);
+            up(P.rank_of, H.rank_of);
+            up(P.halo, H.halo);
+            up(P.exp_of, H.exp_of);
+            const int gl = geom().sms * 8;
+            if (P.g.mask8()) {
+                P.mask8.alloc(P.g.slots());
+                auto kern = upper ? k_line_masks<true, uint8_t> : k_line_masks<false, uint8_t>;
+                kern<<<gl, 256, 0, s>>>(P.g, P.patch.p, T.rp_nat.p, T.ci_nat.p, P.mask8.p);
+            } else {
+                P.mask32.alloc(P.g.slots());
+                auto kern = upper ? k_line_masks<true, uint32_t> : k_line_masks<false, uint32_t>;
+                kern<<<gl, 256, 0, s>>>(P.g, P.patch.p, T.rp_nat.p, T.ci_nat.p, P.mask32.p);
+            }
+            check_launch();
+            XS_CUDA(cudaStreamSynchronize(s));  // the host tables go out of scope
+        } else if (on_grid && want_tiles) {
             auto shrink = [&]() {
                 int &big = tt.tx >= tt.ty && tt.tx >= tt.tz ? tt.tx : (tt.ty >= tt.tz ? tt.ty : tt.tz);
                 if (big <= 2) return false;
@@ -1108,7 +1184,15 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
             }
         }
     }
-    if (T.tiled) {
+    if (T.lined) {
+        T.perm.free(); T.prp.free(); T.pci.free(); T.src.free(); T.lstart.free();
+        if (need_levels) {
+            level_analysis();
+            T.nlevels = P.nlevels;
+            T.lvperm.alloc(n); T.lvperm.upload(P.perm.data(), n, s);
+            XS_CUDA(cudaStreamSynchronize(s));
+        }
+    } else if (T.tiled) {
         Trace tr_bu("      box uploads", s);
         T.ntiles = TP.ntiles;
         T.tile_elems = TP.max_rows + TP.max_halo;
@@ -1606,12 +1690,19 @@ inline void launch_lu_block(const TriDev &L, const TriDev &U, const DT *dinv, co
                                                               U.lstart.p, U.nlevels, dinv, x, z, done_flag);
 }
 
+// reset_other: the other triangle's readiness buffer, re-armed on the way
+// (null when that triangle is line-scheduled and polls no such buffer);
+// X: the exchange buffer of a line-scheduled T, which writes its result to
+// out_user, or to self without one
 template <typename VT, typename FT, typename DT, bool UPPER>
 inline void launch_trsv(const TriDev &T, const DT *dinv, const VT *rhs, VT *self, VT *out_user, VT *reset_other,
-                        const int *done_flag, int *err, cudaStream_t s)
+                        const int *done_flag, int *err, cudaStream_t s, LineXchg<VT> &X)
 {
     const int bo = trsv_tuning().backoff_ns;
-    if (T.tiled) {
+    if (T.lined) {
+        launch_trsv_lines<VT, FT, DT, UPPER, 1>(T.lines, T.vals<FT>(), dinv, X, 1, rhs, out_user ? out_user : self,
+                                                reset_other, done_flag, err, s);
+    } else if (T.tiled) {
         static size_t attr = 0;  // largest dynamic shared memory enabled so far for this instantiation
         const size_t smem = TileSmem::of<VT, FT, DT>(T.t_max_rows, T.t_max_halo, T.t_max_entries).total;
         if (smem > attr) {

@@ -81,6 +81,8 @@ struct TileTuning {
     int min_rows = 65536;
     int blocks_per_sm = 4;
     int user_box = 0;  // tx/ty/tz set by the caller (xs_set_trsv_tiles, XS_TRSV_TILES): no dense-row default
+    int lines = 1;  // line schedule where the pattern qualifies: 1 unless the caller set a box size, 2 also then
+    int line_min_rows = 512;
 };
 // Triangles with at least this many entries per row on average start from
 // TILE_DENSE_BOX boxes instead of tx/ty/tz: small boxes, long along x, four
@@ -220,6 +222,7 @@ inline int grid_reach(int n, const int *rp, const int *ci, LogF logical, const G
 struct TileGrid {
     GridCoord g{0, 0};
     int nx = 0, ny = 0, nz = 0, sa = 0, sb = 0, sc = 0;
+    std::vector<int> vecs;  // the distinct dependency vectors (dx, dy, dz in logical coordinates)
 };
 
 inline bool tile_detect(int n, const int *rp, const int *ci, bool upper, TileGrid &G)
@@ -324,6 +327,7 @@ inline bool tile_detect(int n, const int *rp, const int *ci, bool upper, TileGri
     G.ny = (int)(g.nxy / g.nx);
     G.nz = (int)(n / g.nxy);
     G.sa = sa; G.sb = sb; G.sc = sc;
+    G.vecs.swap(vecs);
     return true;
 }
 

@@ -283,6 +283,7 @@ long max_col_offset(int n, const int *rp, const int *ci)
 void operator_build_ell(Operator &op, const int *rp0, const int *ci0, const double *v, int, bool want32, cudaStream_t s)
 {
     int n = op.n, w = 0;
+    op.layout = next_layout_id();
     for (int i = 0; i < n; i++) w = std::max(w, rp0[i + 1] - rp0[i]);
     const long ld = ell_ld(n);
     const std::vector<int> offs = dia_offsets(n, rp0, ci0);

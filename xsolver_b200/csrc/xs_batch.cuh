@@ -578,8 +578,10 @@ struct BatchPcg {
         };
         // capture a chunk of iterations into a graph and replay it until
         // every column is done (the host polls all_done one chunk behind)
-        std::vector<const void *> key{B, X, R, Z, P, AP, st, ad, &M, A.v, (const void *)(long)k,
-                                      (const void *)(long)M.type};
+        std::vector<const void *> key{B, X, R, Z, P, AP, st, ad, &M, A.rp, A.ci, A.v, (const void *)(long)A.nnz,
+                                      (const void *)(long)k, (const void *)(long)M.type, BP.lb.p, BP.ub.p, BP.lx.x.p,
+                                      BP.ux.x.p};
+        M.graph_key(key);
         if (!gc.exec || gc.key != key) {
             gc.reset();
             cudaGraph_t g;

@@ -20,6 +20,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <mutex>
 #include <thread>
@@ -282,6 +283,17 @@ struct DBuf {
     }
     operator T *() const { return p; }
 };
+
+// Identity of a set of device buffers and the launch parameters that go with
+// them, unique over the process.  A structure whose kernels are captured into
+// graphs takes a new one whenever it is rebuilt, so that a graph captured for
+// the old buffers is never replayed (the address of the structure, or of one
+// of its buffers, can be the same again).
+inline const void *next_layout_id()
+{
+    static std::atomic<uintptr_t> id(0);
+    return (const void *)(++id);
+}
 
 // ---------------------------------------------------------------- device status
 // status word bits written by kernels (device side), read by the host after a

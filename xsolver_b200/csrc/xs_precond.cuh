@@ -88,6 +88,20 @@ struct PrecondDev {
         check_launch();
     }
 
+    // what a captured apply was launched with
+    void graph_key(std::vector<const void *> &key) const
+    {
+        L.graph_key(key);
+        U.graph_key(key);
+        for (const void *q : {(const void *)jdiag64.p, (const void *)jdiag32.p, (const void *)lbuf64.p,
+                              (const void *)ubuf64.p, (const void *)lbuf32.p, (const void *)ubuf32.p,
+                              (const void *)tmp64a.p, (const void *)tmp64b.p, (const void *)tmp64c.p,
+                              (const void *)tmp32a.p, (const void *)tmp32b.p, (const void *)tmp32c.p,
+                              (const void *)lx64.x.p, (const void *)ux64.x.p, (const void *)lx32.x.p,
+                              (const void *)ux32.x.p})
+            key.push_back(q);
+    }
+
     template <typename VT>
     VT *lbuf() const;
     template <typename VT>

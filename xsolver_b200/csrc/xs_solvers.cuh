@@ -92,9 +92,13 @@ inline long cfg_key(const SolveCtx &c)
 
 // Capture `body` `reps` times into a graph and replay until done.
 template <class Body>
-inline void run_graph_loop(SolveCtx &c, GraphCache &gc, const std::vector<const void *> &key, int reps,
-                           int max_launches, Body body)
+inline void run_graph_loop(SolveCtx &c, GraphCache &gc, std::vector<const void *> key, int reps, int max_launches,
+                           Body body)
 {
+    // the operator's and the preconditioner's buffers as well: they are
+    // replaced by a new matrix, a rebuilt factor or a rebuilt transpose
+    c.A->graph_key(key);
+    c.M->graph_key(key);
     if (!gc.exec || gc.key != key) {
         Trace tr("graph capture", c.s);
         gc.reset();

@@ -547,6 +547,15 @@ struct Operator {
     DBuf<float> ev32;
     int ell_grid = 0;
     int *err = nullptr;  // device status word
+    const void *layout = next_layout_id();  // changes with every rebuilt copy below
+    // what a captured kernel of this operator was launched with
+    void graph_key(std::vector<const void *> &key) const
+    {
+        for (const void *q : {layout, (const void *)rp.p, (const void *)ci.p, (const void *)v.p, (const void *)v32.p,
+                              (const void *)tile64.rb.p, (const void *)tile32.rb.p, (const void *)ev.p,
+                              (const void *)ev32.p, (const void *)(long)format})
+            key.push_back(q);
+    }
 
     CsrTileArgs<double> csr64() const
     {

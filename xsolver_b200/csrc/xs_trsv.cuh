@@ -860,6 +860,17 @@ struct TriDev {
     long nnz = 0;
     int nlevels = 0;
     bool upper = false;
+    const void *layout = nullptr;  // changes with every rebuilt analysis
+    // what a captured solve of this triangle was launched with
+    void graph_key(std::vector<const void *> &key) const
+    {
+        for (const void *q : {layout, (const void *)pv64.p, (const void *)pv32.p, (const void *)pvbf.p,
+                              (const void *)pvh.p, (const void *)nv64.p, (const void *)nv32.p, (const void *)nvbf.p,
+                              (const void *)nvh.p, (const void *)ev64.p, (const void *)ev32.p, (const void *)evbf.p,
+                              (const void *)evh.p, (const void *)dinv64.p, (const void *)dinv32.p,
+                              (const void *)dinv64_nat.p, (const void *)dinv32_nat.p})
+            key.push_back(q);
+    }
     DBuf<int> perm, prp, pci;
     DBuf<long> src;
     DBuf<int> lstart;            // level-ordered layout: first position of each level
@@ -1078,6 +1089,7 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
     Trace tr_up("    upload + positions", s);
     Trace tr_nat("      natural CSR + sources", s);
     T.n = n;
+    T.layout = next_layout_id();
     T.nnz = rp[n];
     T.nlevels = -1;
     T.upper = upper;

@@ -473,6 +473,11 @@ int xs_set_trsv_tiles(int enable, int tx, int ty, int tz, int min_rows);
  * 2 also with a box size set; 0 never.  Results are bitwise the same.
  * Fixed when a preconditioner is built. */
 int xs_set_trsv_lines(int mode, int min_rows);
+/* Exact LU solves of patterns without a grid schedule on one thread-block
+ * cluster, the solution vector in its distributed shared memory (FP64 up to
+ * about 450,000 rows): 1 (default), or 0 for the sync-free solve through
+ * global memory.  Results are bitwise the same. */
+int xs_set_trsv_cluster(int enable);
 /* Exact LU solves of systems with at most max_rows rows, whose solution
  * vector fits in one SM's shared memory (FP64: 25600 rows), run in one CTA
  * that walks the dependency levels with a block barrier between them

@@ -103,6 +103,7 @@ def _declare(L):
         "xs_set_trsv_tiles": [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int],
         "xs_tri_lines": [C.c_int, _ip, _ip, C.c_int, *([_ip] * 8)],
         "xs_set_trsv_lines": [C.c_int, C.c_int],
+        "xs_set_trsv_cluster": [C.c_int],
         "xs_tri_tiles": [C.c_int, _ip, _ip, C.c_int, C.c_int, C.c_int, C.c_int, _ip, _ip, _ip, _ip, _ip, _ip, _ip,
                          _ip, _ip],
         "xs_set_ell_index_bits": [C.c_int],

@@ -2000,6 +2000,11 @@ int xs_tri_lines(int n, const int *rp, const int *ci, int upper, int *info, int 
     });
 }
 
+int xs_set_trsv_cluster(int enable)
+{
+    return guarded([&] { trsv_tuning().cluster = enable != 0; });
+}
+
 int xs_set_trsv_lines(int mode, int min_rows)
 {
     return guarded([&] {

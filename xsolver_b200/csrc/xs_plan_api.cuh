@@ -302,14 +302,19 @@ int xs_plan_debug_break_dependency(xs_plan_t p, int position, int enable)
         int row = 0;
         XS_CUDA(cudaMemcpy(&row, L.perm.p + position, sizeof(int), cudaMemcpyDeviceToHost));
         // the saved entry may be an encoded (negative) chunk-local slot
-        static thread_local int saved = 0;
+        static thread_local int saved = 0, saved_pos = 0;
         static thread_local bool have_saved = false;
         if (enable) {
-            if (!have_saved) XS_CUDA(cudaMemcpy(&saved, L.pci.p + k[0], sizeof(int), cudaMemcpyDeviceToHost));
+            if (!have_saved) {
+                XS_CUDA(cudaMemcpy(&saved, L.pci.p + k[0], sizeof(int), cudaMemcpyDeviceToHost));
+                if (L.ppos.p) XS_CUDA(cudaMemcpy(&saved_pos, L.ppos.p + k[0], sizeof(int), cudaMemcpyDeviceToHost));
+            }
             have_saved = true;
             XS_CUDA(cudaMemcpy(L.pci.p + k[0], &row, sizeof(int), cudaMemcpyHostToDevice));  // waits on itself
+            if (L.ppos.p) XS_CUDA(cudaMemcpy(L.ppos.p + k[0], &position, sizeof(int), cudaMemcpyHostToDevice));
         } else if (have_saved) {
             XS_CUDA(cudaMemcpy(L.pci.p + k[0], &saved, sizeof(int), cudaMemcpyHostToDevice));
+            if (L.ppos.p) XS_CUDA(cudaMemcpy(L.ppos.p + k[0], &saved_pos, sizeof(int), cudaMemcpyHostToDevice));
             have_saved = false;
         }
     });

@@ -43,6 +43,8 @@ struct PrecondDev {
     DBuf<float> lbuf32, ubuf32, tmp32a, tmp32b, tmp32c;
     LineXchg<double> lx64, ux64;  // exchange buffers of line-scheduled solves
     LineXchg<float> lx32, ux32;
+    DBuf<double> y64;  // L's result inside the cluster solve
+    DBuf<float> y32;
     int *err = nullptr;
     bool have_factors = false;
 
@@ -57,6 +59,7 @@ struct PrecondDev {
         }
         if (L.lined) line_xchg_ensure(lx64, L.lines.g, 1, s);
         if (U.lined) line_xchg_ensure(ux64, U.lines.g, 1, s);
+        if (L.ppos.p && y64.n != (size_t)n) y64.alloc(n);
     }
     void ensure_buffers32(cudaStream_t s)
     {
@@ -69,6 +72,7 @@ struct PrecondDev {
         }
         if (L.lined) line_xchg_ensure(lx32, L.lines.g, 1, s);
         if (U.lined) line_xchg_ensure(ux32, U.lines.g, 1, s);
+        if (L.ppos.p && y32.n != (size_t)n) y32.alloc(n);
     }
     // temporaries of the Jacobi-sweep mode
     void ensure_sweep_buffers(bool need32)
@@ -98,7 +102,7 @@ struct PrecondDev {
                               (const void *)tmp64a.p, (const void *)tmp64b.p, (const void *)tmp64c.p,
                               (const void *)tmp32a.p, (const void *)tmp32b.p, (const void *)tmp32c.p,
                               (const void *)lx64.x.p, (const void *)ux64.x.p, (const void *)lx32.x.p,
-                              (const void *)ux32.x.p})
+                              (const void *)ux32.x.p, (const void *)y64.p, (const void *)y32.p})
             key.push_back(q);
     }
 
@@ -106,6 +110,8 @@ struct PrecondDev {
     VT *lbuf() const;
     template <typename VT>
     VT *ubuf() const;
+    template <typename VT>
+    VT *ybuf() const;
 
     // z = M^{-1} x on stream s.  x == z allowed.
     template <typename VT>
@@ -152,6 +158,14 @@ struct PrecondDev {
             if constexpr (std::is_same<VT, double>::value) dinv = U.dinv64.p;
             else dinv = U.dinv32.p;
             launch_lu_block<VT, FT, VT>(L, U, dinv, x, z, done_flag, s);
+            return;
+        }
+        if (const int slots = lu_cluster_slots<VT, FT, VT>(L, U)) {
+            const VT *dinv;
+            if constexpr (std::is_same<VT, double>::value) dinv = U.dinv64.p;
+            else dinv = U.dinv32.p;
+            // y goes to a buffer of its own: lbuf stays armed for the halves
+            launch_lu_cluster<VT, FT, VT>(L, U, slots, dinv, x, ybuf<VT>(), z, done_flag, err, s);
             return;
         }
         exact_half<VT, FT>(0, x, z, done_flag, s);
@@ -347,6 +361,10 @@ struct PrecondDev {
 
 template <>
 inline double *PrecondDev::lbuf<double>() const { return lbuf64.p; }
+template <>
+inline double *PrecondDev::ybuf<double>() const { return y64.p; }
+template <>
+inline float *PrecondDev::ybuf<float>() const { return y32.p; }
 template <>
 inline double *PrecondDev::ubuf<double>() const { return ubuf64.p; }
 template <>

@@ -137,6 +137,9 @@ struct TrsvTuning {
     // 128^2 231 us with 768-row batches against 234 at 512 and 260-311 with
     // 3-4 smaller buffers)
     int lub_rows = 512, lub_entries = 2048, lub_bufs = 2, lub_auto = 1;
+    // exact LU solve on one thread-block cluster (k_lu_cluster) where the
+    // solution fits in its shared memory; 0 keeps the sync-free solve
+    int cluster = 1;
     // Jacobi-sweep passes on a grid whose CTAs all take the same number of
     // row blocks (1) or on one full wave of CTAs (0)
     int balanced_sweep_grid = 0;
@@ -407,7 +410,8 @@ __global__ void k_fill_sentinel(VT *b, int n)
 
 }  // namespace xs
 
-#include "xs_trsv_lines.cuh"  // line-scheduled exact solves (uses msub, k_fill_sentinel)
+#include "xs_trsv_lines.cuh"    // line-scheduled exact solves (uses msub, k_fill_sentinel)
+#include "xs_trsv_cluster.cuh"  // exact LU solve on one cluster
 
 namespace xs {
 
@@ -916,6 +920,7 @@ struct TriDev {
     int lub_rows = 0, lub_entries = 0;  // batch limits the list was built with
     int max_level_rows = 0;  // widest dependency level (level layout)
     DBuf<int> lub;
+    DBuf<int> ppos;  // level layout: dependency position of each entry (k_lu_cluster)
     bool tiled = false;
     int ntiles = 0, tile_elems = 0;  // tile_elems: shared-memory values per box (rows + halo)
     int t_max_rows = 0, t_max_halo = 0, t_max_entries = 0;
@@ -1252,6 +1257,16 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
         k_pos_entries<<<g, 256, 0, s>>>(n, upper, T.perm.p, T.prp.p, T.rp_nat.p, T.ci_nat.p, T.src_nat.p, T.pci.p,
                                         T.src.p);
         check_launch();
+        T.ppos.free();
+        if (T.nnz && n <= CLU_MAX * (int)(CLU_SMEM_MAX / sizeof(float))) {  // sizes the cluster solve can serve
+            DBuf<int> pos_of;
+            pos_of.alloc(n);
+            T.ppos.alloc(m);
+            k_inverse_perm<<<g, 256, 0, s>>>(n, T.perm.p, pos_of.p);
+            k_entry_positions<<<g, 256, 0, s>>>(T.nnz, T.pci.p, pos_of.p, T.ppos.p);
+            check_launch();
+            XS_CUDA(cudaStreamSynchronize(s));  // before the temporary is freed
+        }
         T.lstart.alloc(P.nlevels + 1, 4); T.lstart.upload(P.lstart.data(), P.nlevels + 1, s);
         T.max_level_rows = 0;
         for (int l = 0; l < P.nlevels; l++) T.max_level_rows = std::max(T.max_level_rows, P.lstart[l + 1] - P.lstart[l]);
@@ -1700,6 +1715,47 @@ inline void launch_lu_block(const TriDev &L, const TriDev &U, const DT *dinv, co
     }
     k_lu_block<VT, FT, DT><<<1, LU_BLOCK_THREADS, smem, s>>>(L.args<FT>(), L.lstart.p, L.nlevels, U.args<FT>(),
                                                               U.lstart.p, U.nlevels, dinv, x, z, done_flag);
+}
+
+// whether the cluster solve serves this pair of plans for vectors of VT, as
+// its slots per CTA (0: no)
+template <typename VT, typename FT, typename DT>
+inline int lu_cluster_slots(const TriDev &L, const TriDev &U)
+{
+    if (!trsv_tuning().cluster || !L.ppos.p || !U.ppos.p) return 0;
+    const int C = clu_size<VT, FT, DT>();
+    if (C == 0) return 0;
+    const int groups = (L.n + 31) / 32, slots = (groups + C - 1) / C * 32;
+    return (size_t)slots * sizeof(VT) <= CLU_SMEM_MAX ? slots : 0;
+}
+
+template <typename VT, typename FT, typename DT>
+inline void launch_lu_cluster(const TriDev &L, const TriDev &U, int slots, const DT *dinv, const VT *x, VT *y, VT *z,
+                              const int *done_flag, int *err, cudaStream_t s)
+{
+    const int C = clu_size<VT, FT, DT>();
+    int cshift = 0;
+    while ((1 << cshift) < C) cshift++;
+    // about CLU_AHEAD levels' rows in flight
+    const long width = std::max(1L, (long)L.n / std::max(1, std::max(L.nlevels, U.nlevels)));
+    const int nw = (int)std::max(1L, std::min<long>(CLU_WARPS_MAX, (CLU_AHEAD * width + 32 * C - 1) / (32 * C)));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(32 * nw);
+    cfg.dynamicSmemBytes = (size_t)slots * sizeof(VT);
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = pdl_tuning().enabled ? 1 : 0;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    if (cudaLaunchKernelEx(&cfg, k_lu_cluster<VT, FT, DT>, L.args<FT>(), (const int *)L.ppos.p, U.args<FT>(),
+                           (const int *)U.ppos.p, dinv, x, y, z, done_flag, err, (uint32_t)C, (uint32_t)cshift,
+                           slots) != cudaSuccess)
+        throw Status(XS_ERR_CUDA);
 }
 
 // reset_other: the other triangle's readiness buffer, re-armed on the way

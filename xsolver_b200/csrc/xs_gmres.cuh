@@ -52,6 +52,32 @@ __device__ inline void gm_genrot(double dx, double dy, double &cs, double &sn)
     }
 }
 
+// the end of step i (one thread): tot = (w, w) after the last subtraction;
+// completes H's column, rotates it and tests for convergence
+__device__ inline void gm_norm_finish(KState *st, const GmDev &g, int i, int quirk, double tot)
+{
+    const int m = g.m;
+    double *H = g.H;
+    const double nrm = sqrt(tot);
+    H[(i + 1) * m + i] = nrm;
+    st->sc[S_GM_INV] = 1.0 / (nrm + KSMALL);
+    for (int k = 0; k < i; k++) gm_applyrot(H[k * m + i], H[(k + 1) * m + i], g.cs[k], g.sn[k]);
+    gm_genrot(H[i * m + i], H[(i + 1) * m + i], g.cs[i], g.sn[i]);
+    gm_applyrot(H[i * m + i], H[(i + 1) * m + i], g.cs[i], g.sn[i]);
+    gm_applyrot(g.s[i], g.s[i + 1], g.cs[i], g.sn[i]);
+    const bool cont = record_and_test(st, fabs(g.s[i + 1]));
+    if (!cont) {
+        if (st->done == 1) st->kcols = quirk ? i : i + 1;
+        else st->kcols = i + 1;
+    }
+}
+
+}  // namespace xs
+
+#include "xs_gmres_orth.cuh"  // a step's orthogonalisation in one kernel (uses gm_norm_finish)
+
+namespace xs {
+
 // w = w - h V_prev ; last step of MGS, acc = w.w, then Givens (thread 0 of last block)
 template <typename VT>
 struct OpGmNorm {
@@ -73,23 +99,7 @@ struct OpGmNorm {
         w[q] = wi;
         a[0] += (double)wi * (double)wi;
     }
-    __device__ void finalize(const double *t) const
-    {
-        const int m = g.m;
-        double *H = g.H;
-        const double nrm = sqrt(t[0]);
-        H[(i + 1) * m + i] = nrm;
-        st->sc[S_GM_INV] = 1.0 / (nrm + KSMALL);
-        for (int k = 0; k < i; k++) gm_applyrot(H[k * m + i], H[(k + 1) * m + i], g.cs[k], g.sn[k]);
-        gm_genrot(H[i * m + i], H[(i + 1) * m + i], g.cs[i], g.sn[i]);
-        gm_applyrot(H[i * m + i], H[(i + 1) * m + i], g.cs[i], g.sn[i]);
-        gm_applyrot(g.s[i], g.s[i + 1], g.cs[i], g.sn[i]);
-        const bool cont = record_and_test(st, fabs(g.s[i + 1]));
-        if (!cont) {
-            if (st->done == 1) st->kcols = quirk ? i : i + 1;
-            else st->kcols = i + 1;
-        }
-    }
+    __device__ void finalize(const double *t) const { gm_norm_finish(st, g, i, quirk, t[0]); }
 };
 
 // dst = src * scale (scale from a KState slot)
@@ -170,12 +180,14 @@ struct GmresRun {
     VecPool<VT> pool;
     DBuf<VT> V, Z;
     DBuf<double> gm;
+    DBuf<unsigned> bar;  // grid barrier of the one-kernel orthogonalisation
     int mcap = 0;
     GraphCache gc;
     void run(SolveCtx &c, const VT *b, VT *x, int m, bool right)
     {
         const int n = c.n;
         if (m < 1) m = 1;
+        if (!bar.p) bar.alloc(2);
         if (mcap != m || V.n != (size_t)(m + 1) * n) {
             V.alloc((size_t)(m + 1) * n);
             if (right) Z.alloc((size_t)(m + 1) * n);
@@ -205,6 +217,11 @@ struct GmresRun {
         if (!right) c.M->apply<VT>(res, res, nullptr, c.s);
         vecop(OpGmInit<VT>{n, st, res}, sl, c.s);
         const int quirk = c.quirk;
+        // a step's orthogonalisation in one cooperative launch where w fits in
+        // the registers of one CTA per SM, else one launch per coefficient
+        const OrthShape<VT> orth = orth_shape<VT>(n);
+        if (orth.grid) XS_CUDA(cudaMemsetAsync(bar.p, 0, 2 * sizeof(unsigned), c.s));  // also after an aborted solve
+        const GridBar gb{bar.p, c.M->err};
         auto cycle = [&]() {
             k_gm_cycle_init<<<1, 256, 0, c.s>>>(st, g);
             vecop(OpScaleCopy<VT>{n, st, Vk(0), res, S_GM_INV, 1, (VT)0}, sl, c.s);
@@ -215,6 +232,10 @@ struct GmresRun {
                 } else {
                     spmv<VT, MT>(*c.A, Vk(i), w, EpiActive<VT>{st}, sl, c.s);
                     c.M->apply<VT>(w, w, done, c.s);
+                }
+                if (orth.grid) {
+                    launch_gm_orth<VT>(orth, n, st, w, V.p, g, i, quirk, sl.part, gb, c.s);
+                    continue;
                 }
                 // h_0 = w.V_0
                 vecop(OpMgsStep<VT>{n, st, w, nullptr, Vk(0), nullptr, &g.H[0 * m + i], (VT)0}, sl, c.s);

@@ -185,3 +185,58 @@ def test_infinities_and_nans_pass_through(cuda):
     with lines_mode(2):
         (z,) = _lusolve(Plan(A).factor("ilu0"), x, cuda)
     assert np.array_equal(z, oracle.lusolve(F, x), equal_nan=True)
+
+
+@pytest.mark.parametrize("shape", [(9, 11, 10), (17, 33, 9), (40, 41, 42), (33, 17, 71), (129, 63), (7, 300), (128, 128)])
+def test_ilu0_on_lines_bitwise_vs_oracle(cuda, shape):
+    """ILU(0) of 5- and 7-point patterns on the line schedule: the reference's
+    factors bit for bit, also where an entry has no transposed one, and a
+    pivot near zero takes the reference's substitute."""
+    from xsolver_b200 import CSRMatrix
+    from xsolver_b200.api import Plan
+
+    A = _stencil(shape, P7 if len(shape) == 3 else P5, 3)
+    rows = np.repeat(np.arange(A.n), np.diff(A.rowptr))
+    rng = np.random.default_rng(5)
+    for M in (A, None):
+        if M is None:  # one-sided couplings, and a first pivot of zero
+            keep = (A.colidx == rows) | (rng.random(A.nnz) < 0.96)
+            rp = np.zeros(A.n + 1, np.int64)
+            np.cumsum(np.bincount(rows[keep], minlength=A.n), out=rp[1:])
+            M = CSRMatrix(A.n, rp, A.colidx[keep], A.val[keep])
+            M.val[0] = 0.0
+        with lines_mode(2):
+            P = Plan(M).factor("ilu0")
+            assert np.array_equal(P.lu_values(), oracle.ilu0_values(M))
+            assert np.array_equal(P.factor("ilu0").lu_values(), oracle.ilu0_values(M))  # refactorised
+
+
+def test_repeated_columns_keep_their_order(cuda):
+    """A row with the same column twice is solved by a schedule that keeps both entries."""
+    from xsolver_b200 import CSRMatrix
+    from xsolver_b200.api import Plan
+
+    A = _stencil((12, 13, 14), P7, 1)
+    e = int(A.rowptr[700])  # repeat the first (lower) entry of row 700
+    ci, v = np.insert(A.colidx, e, A.colidx[e]), np.insert(A.val, e, -0.25)
+    rp = A.rowptr.copy()
+    rp[701:] += 1
+    B = CSRMatrix(A.n, rp, ci, v)
+    x = st.rhs_uniform(A.n, 1)
+    with lines_mode(2):
+        P = Plan(B).factor("ilu0")
+        (z,) = _lusolve(P, x, cuda)
+        F = P.factors()
+    y = np.zeros(A.n)
+    for r in range(A.n):
+        acc = x[r]
+        for q in range(F["lrp"][r], F["lrp"][r + 1]):
+            acc = acc - y[F["lci"][q]] * F["lv"][q]
+        y[r] = acc
+    w = np.zeros(A.n)
+    for r in range(A.n - 1, -1, -1):
+        acc = y[r] * F["dinv"][r]
+        for q in range(F["urp"][r + 1] - 1, F["urp"][r] - 1, -1):
+            acc = acc - w[F["uci"][q]] * F["uv"][q]
+        w[r] = acc
+    assert np.array_equal(z, w)

@@ -422,6 +422,10 @@ struct Handle {
     size_t ilu_tiles_smem = 0;
     int ilu_max_entries = 0, ilu_max_lower = 0, ilu_max_rows = 0;
     DBuf<int> ilu_ebase, ilu_ent, ilu_roff, ilu_rdiag, ilu_lbase, ilu_loff, ilu_dep;
+    // ILU(0) on the line schedule of the L solve (line_ilu_ok)
+    DBuf<double> lilu_pv, lilu_a, lilu_d;
+    DBuf<uint8_t> lilu_mask;
+    LineXchg<double> lilu_x;
     TriHostPlan hL, hU;
     DBuf<double> luv, fv, tmpv;
     DBuf<long> udiag_src;
@@ -882,7 +886,7 @@ static void factor_ic0(Handle &h)
     analyse_pattern(h);
     ensure_ic0_maps(h);
     const int n = h.n;
-    h.luv.alloc(std::max<long>(h.nnz, 1));
+    if (h.luv.n != (size_t)std::max<long>(h.nnz, 1)) h.luv.alloc(std::max<long>(h.nnz, 1));
     XS_CUDA(cudaMemcpyAsync(h.luv.p, h.A.v.p, sizeof(double) * h.nnz, cudaMemcpyDeviceToDevice, h.s));
     k_ic0_tnorm<<<geom().sms * 4, 256, 0, h.s>>>(n, h.A.rp.p, h.A.v.p, IC0_DROPTOL, h.ic0_tnorm.p);
     h.ilu_epoch++;
@@ -905,7 +909,7 @@ static void factor_ilu(Handle &h, int kind, int sweeps)
 {
     analyse_pattern(h);
     const int n = h.n;
-    h.luv.alloc(std::max<long>(h.nnz, 1));
+    if (h.luv.n != (size_t)std::max<long>(h.nnz, 1)) h.luv.alloc(std::max<long>(h.nnz, 1));
     XS_CUDA(cudaMemcpyAsync(h.luv.p, h.A.v.p, sizeof(double) * h.nnz, cudaMemcpyDeviceToDevice, h.s));
     if (kind == 0) {
         h.ilu_epoch++;
@@ -942,6 +946,9 @@ static void factor_ilu(Handle &h, int kind, int sweeps)
         const int wmax = h.max_row_len;
         int G = 4;
         while (G < wmax && G < 64) G <<= 1;
+        const TriDev &TL = h.M.L;
+        const bool on_lines = TL.lined && h.M.U.lined && h.nnz == TL.nnz + h.M.U.nnz + n &&  // one diagonal entry a row
+                              line_ilu_ok(TL.lines, h.M.U.lines);
         if (ilu_tiles_flag() && !h.ilu_tiles_built) {
             build_ilu_tiles(h);
             h.ilu_tiles_built = true;
@@ -963,6 +970,27 @@ static void factor_ilu(Handle &h, int kind, int sweeps)
                                    h.ilu_epoch, h.err.p, h.fticket.p};
             k_ilu0_tiles<<<gl, ILU_TILE_THREADS, sm, h.s>>>(args, h.ilu_max_entries, h.ilu_max_lower,
                                                             h.ilu_max_rows);
+        } else if (on_lines) {
+            const LinePlan &P = TL.lines;
+            const size_t m = (size_t)P.g.slots();
+            if (h.lilu_mask.n != m) {
+                h.lilu_mask.alloc(m);
+                h.lilu_pv.alloc(m * 2 * P.g.D);
+            }
+            if (h.lilu_a.n != (size_t)n) {
+                h.lilu_a.alloc(n);
+                h.lilu_d.alloc(n);
+            }
+            line_xchg_ensure(h.lilu_x, P.g, 1, h.s);
+            const int g8 = geom().sms * 8;
+            k_line_pairs<<<g8, 256, 0, h.s>>>(P.g, P.patch.p, h.A.rp.p, h.A.ci.p, h.uptr.p, h.A.v.p, h.lilu_pv.p,
+                                              h.lilu_mask.p);
+            k_line_diag<<<g8, 256, 0, h.s>>>(n, h.uptr.p, h.A.v.p, h.lilu_a.p);
+            check_launch();
+            launch_trsv_lines<double, double, double, false, 1, true>(P, h.lilu_pv.p, h.lilu_mask.p,
+                                                                      (const double *)nullptr, h.lilu_x, 1, h.lilu_a.p,
+                                                                      h.lilu_d.p, (double *)nullptr, nullptr, h.err.p, h.s);
+            k_line_ilu_finish<<<g8, 256, 0, h.s>>>(n, h.A.rp.p, h.A.ci.p, h.uptr.p, h.lilu_d.p, h.luv.p);
         } else if (ilu_group && G <= 32) {
             const int rpb = 128 / G;
             const int bps = ilu_bps_env ? ilu_bps_env : (G <= 8 ? 4 : 8);
@@ -983,7 +1011,7 @@ static void factor_ilu(Handle &h, int kind, int sweeps)
         check_launch();
     } else {
         ensure_entry_maps(h, true);
-        h.tmpv.alloc(std::max<long>(h.nnz, 1));
+        if (h.tmpv.n < (size_t)std::max<long>(h.nnz, 1)) h.tmpv.alloc(std::max<long>(h.nnz, 1));
         const int g = geom().sms * 8;
         double *cur = h.luv.p, *nxt = h.tmpv.p;
         for (int sw = 0; sw < sweeps; sw++) {
@@ -996,7 +1024,10 @@ static void factor_ilu(Handle &h, int kind, int sweeps)
             XS_CUDA(cudaMemcpyAsync(h.luv.p, cur, sizeof(double) * h.nnz, cudaMemcpyDeviceToDevice, h.s));
     }
     int e = read_dev_err(h);
-    if (e) throw Status(dev_err_to_status(e));
+    if (e) {
+        line_xchg_rearm(h.lilu_x, h.s);
+        throw Status(dev_err_to_status(e));
+    }
 }
 
 // host-computed factors (L strict, dinv, U' strict) into the device layout

@@ -1132,6 +1132,16 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
     const bool want_lines = !T.chunked && tile_tuning().enable && n >= tile_tuning().line_min_rows &&
                             (tile_tuning().lines == 2 || (tile_tuning().lines && !tile_tuning().user_box));
     const bool want_tiles = !T.chunked && tile_tuning().enable && n >= tile_tuning().min_rows;
+    // a row with the same column twice has no place for its second entry on
+    // the diagonals (columns are sorted, so repeats are neighbours)
+    auto repeats = [&]() {
+        std::vector<char> seen(16, 0);
+        host_parallel_rows(n, [&](long lo, long hi, int t) {
+            for (long i = lo; i < hi; i++)
+                for (int k = rp[i] + 1; k < rp[i + 1]; k++) seen[t] |= ci[k] == ci[k - 1];
+        });
+        return std::find(seen.begin(), seen.end(), 1) != seen.end();
+    };
     if (want_lines || want_tiles) {
         Trace tr_tile("    grid analysis", s);
         TileTuning tt = tile_tuning();
@@ -1140,7 +1150,7 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
         Trace tr_det("      grid detection", s);
         const bool on_grid = tile_detect(n, rp.data(), ci.data(), upper, G);
         tr_det.stop();
-        if (on_grid && want_lines && line_layout(n, T.nnz, G, geom().sms, H)) {
+        if (on_grid && want_lines && line_layout(n, T.nnz, G, geom().sms, H) && !repeats()) {
             T.lined = true;
             LinePlan &P = T.lines;
             P.g = H.g;
@@ -1768,7 +1778,7 @@ inline void launch_trsv(const TriDev &T, const DT *dinv, const VT *rhs, VT *self
 {
     const int bo = trsv_tuning().backoff_ns;
     if (T.lined) {
-        launch_trsv_lines<VT, FT, DT, UPPER, 1>(T.lines, T.vals<FT>(), dinv, X, 1, rhs, out_user ? out_user : self,
+        launch_trsv_lines<VT, FT, DT, UPPER, 1>(T.lines, T.vals<FT>(), T.lines.mask8.p, dinv, X, 1, rhs, out_user ? out_user : self,
                                                 reset_other, done_flag, err, s);
     } else if (T.tiled) {
         static size_t attr = 0;  // largest dynamic shared memory enabled so far for this instantiation

@@ -31,17 +31,24 @@
 //                     pattern no arithmetic produces marks a value not yet
 //                     published, every wait bounded) and run ahead of the
 //                     compute threads as far as the ring allows
-//   helper warps      stage the factor data NS stages ahead (one bulk copy
+//   staging warps     bring the factor data NS stages ahead (one bulk copy
 //                     each for values, diagonal and masks, stored in exactly
-//                     the order they are used) and the right-hand side, and
-//                     drain finished steps to the output along x, so that
+//                     the order they are used) and the right-hand side
+//   draining warps    write finished steps to the output along x, so that
 //                     vectors stay in natural order and accesses coalesce
+//
+// Measured on B200, an LU solve in FP64, boxes / lines: 128^3 7-point
+// 932 / 318 us, 80^3 27-point 566 us, 128^2 5-point 90 us (197 us in one
+// CTA), eight right-hand sides at 96^3 415 us.  A 7-point step is about 330
+// cycles, of which the sums are 40 and storing, a barrier and reading back
+// 67; DRAM stays below 20 % of its rate.
 //
 // Patches are taken by ticket in an order in which dependencies come first,
 // so a CTA only waits on patches that running CTAs hold: no co-residency is
 // needed.  The exchange buffer is doubled: a launch publishes into one half
 // and re-arms the other for the next launch.
 #pragma once
+#include <climits>
 #include <vector>
 #include "xs_internal.cuh"
 #include "xs_spmv.cuh"
@@ -50,11 +57,13 @@
 namespace xs {
 
 constexpr int LINE_DIAG_MAX = 32;   // entries per row: bits of the row mask
-constexpr int LINE_PATCH = 128;       // lines per patch
+// lines per patch for D diagonals: a compile-time constant of the kernels.
+// Four warps hide each other's gaps where a step is a few sums; with more
+// diagonals the step is bound by instructions and shared-memory traffic, and
+// twice as many CTAs take it.
+__host__ __device__ constexpr int line_patch(int D) { return D == 2 || D == 3 ? 128 : 64; }
 constexpr int LINE_HALO_MAX = 64;   // halo lines per patch
-constexpr int LINE_HELPERS = 128;   // staging / draining threads
-constexpr int LINE_POLL_WARPS = 4;  // most poller warps
-constexpr int LINE_ITEMS = 2;       // halo values polled per poller lane
+constexpr int LINE_HELPERS = 128;   // staging threads, and as many draining threads
 constexpr int LINE_WINDOW = 8;      // steps polled at once
 constexpr int LINE_STEP = 8;        // steps per patch are a multiple of this (the longest stage)
 constexpr size_t LINE_SMEM_MAX = 222 * 1024;
@@ -68,6 +77,7 @@ struct LineGeo {
     int npy = 0, npz = 0, npatch = 0, nsteps = 0;
     int D = 0, E = 0, nh = 0, maxd = 0;  // diagonals, exported lines, halo lines, longest step distance
     int delta[LINE_DIAG_MAX] = {}, shift[LINE_DIAG_MAX] = {}, offq[LINE_DIAG_MAX] = {};
+    int back[LINE_DIAG_MAX] = {};  // ring distance of a diagonal's value: delta rows and shift columns
     // first logical index of line (Yl, Zl) of patch (pY, pZ), or -1 outside the grid
     __host__ __device__ int line_q0(int pY, int pZ, int Yl, int Zl) const
     {
@@ -85,7 +95,8 @@ constexpr int LINE_NS_MAX = 8;  // most stages
 struct LineSmem {
     size_t ring, rhs, pv, dinv, mask, tab, total;
     int Ps, RS;  // ring columns per step (odd), right-hand-side columns per step (odd)
-    static __host__ __device__ LineSmem of(const LineGeo &g, int S, int NS, int RL, int KC, size_t vb, size_t fb,
+    // nv: values per row in the stream (the diagonals', or twice as many for the factorisation)
+    static __host__ __device__ LineSmem of(const LineGeo &g, int nv, int S, int NS, int RL, int KC, size_t vb, size_t fb,
                                            size_t db, size_t mb)
     {
         auto al = [](size_t b) { return (b + 127) & ~(size_t)127; };
@@ -93,12 +104,12 @@ struct LineSmem {
         m.Ps = g.npad | 1;
         m.RS = (g.L * KC) | 1;
         m.ring = 0;
-        m.rhs = m.ring + al((size_t)RL * m.Ps * KC * vb);
+        m.rhs = m.ring + al((size_t)2 * RL * m.Ps * KC * vb);  // every step twice, RL rows apart
         m.pv = m.rhs + al((size_t)NS * S * m.RS * vb);
-        m.dinv = m.pv + al((size_t)NS * S * g.D * g.L * fb);
+        m.dinv = m.pv + al((size_t)NS * S * nv * g.L * fb);
         m.mask = m.dinv + al((size_t)NS * S * g.L * db);
         m.tab = m.mask + al((size_t)NS * S * g.L * mb);
-        m.total = m.tab + al((size_t)3 * g.L * sizeof(int));
+        m.total = m.tab + al((size_t)g.L * 4 * sizeof(int));
         return m;
     }
 };
@@ -111,7 +122,7 @@ struct LineCfg {
     int S = 0, NS = 0, RL = 0;
     size_t smem = 0;
 };
-inline LineCfg line_cfg(const LineGeo &g, int items, int KC, size_t vb, size_t fb, size_t db, size_t mb, int sms)
+inline LineCfg line_cfg(const LineGeo &g, int nv, int items, int KC, size_t vb, size_t fb, size_t db, size_t mb, int sms)
 {
     LineCfg c;
     int best = -1;
@@ -120,11 +131,11 @@ inline LineCfg line_cfg(const LineGeo &g, int items, int KC, size_t vb, size_t f
             for (int S = LINE_STEP; S >= 1; S /= 2)
                 for (int NS = LINE_NS_MAX; NS >= 3; NS--) {
                     const int ahead = RL - g.maxd - S;  // steps the pollers run ahead
-                    if (ahead < LINE_WINDOW || RL < 2 * S) continue;
-                    const size_t b = LineSmem::of(g, S, NS, RL, KC, vb, fb, db, mb).total;
+                    if (ahead < 8 || RL < 2 * S) continue;
+                    const size_t b = LineSmem::of(g, nv, S, NS, RL, KC, vb, fb, db, mb).total;
                     if (b > lim) continue;
                     if (lim != LINE_SMEM_MAX && NS * S < 12) continue;  // too little in flight to share an SM
-                    const int score = std::min(NS * S, 24) * 10000 + std::min(ahead, 24) * 100 + 10 * S + (8 - NS);
+                    const int score = std::min(NS * S, 24) * 10000 + S * 1000 + std::min(ahead, 16) * 10 + (8 - NS);
                     if (score <= best) continue;
                     best = score;
                     c.S = S; c.NS = NS; c.RL = RL; c.smem = b;
@@ -208,21 +219,24 @@ inline bool line_layout(int n, long nnz, const TileGrid &G, int sms, LineHost &h
     // patches take on the GPU's SMs (microseconds; the constants are the
     // measured step and hand-off of the kernel below, to one digit)
     const int Yext = g.ny + c * (g.nz - 1);
-    const double ts = 0.05 + 0.005 * D, th = 1.0;
     double best = 1e300;
-    for (int L = 32; L <= LINE_PATCH; L *= 2)
+    {
+        const int L = line_patch(D);
         for (int ty = 1; ty <= L; ty *= 2) {
+            const double ts = (100.0 + 20.0 * D) / 1900.0, th = 0.6;
             const int tz = L / ty;
             if (ty < g.ry || tz < g.rz) continue;
             const int npy = (Yext + ty - 1) / ty, npz = (g.nz + tz - 1) / tz;
-            const int ns = (g.nx + al * (ty - 1) + be * (tz - 1) + LINE_STEP - 1) / LINE_STEP * LINE_STEP;
+            // steps of a patch (a patch wider than the domain ends with its last line)
+            const int ns = (g.nx + al * (std::min(ty, Yext) - 1) + be * (std::min(tz, g.nz) - 1) + LINE_STEP - 1) /
+                           LINE_STEP * LINE_STEP;
             // patches that hold lines (the sheared domain is a parallelogram)
             long np = 0;
             for (int p = 0; p < npz; p++) {
                 const int z0 = p * tz, z1 = std::min(g.nz, z0 + tz) - 1;
                 np += (c * z1 + g.ny - 1) / ty - (c * z0) / ty + 1;
             }
-            if (np * ns * L > 4L * n + 16384) continue;  // mostly padding
+            if (np * ns * L > 4L * n + 65536) continue;  // mostly padding
             const double chain = (g.nx + al * (double)(Yext - 1) + be * (double)(g.nz - 1)) * ts + (npy + npz - 2) * th;
             const double stream = (double)np * ns * L * (8.0 * D + 24.0) / 5.5e6;
             const double work = (double)np * ns * ts / sms;
@@ -230,16 +244,20 @@ inline bool line_layout(int n, long nnz, const TileGrid &G, int sms, LineHost &h
             LineGeo t = g;
             t.L = L; t.ty = ty; t.tz = tz;
             t.npad = (ty + g.ry) * (tz + g.rz);
-            if (cost < best && line_cfg(t, 0, 1, 8, 8, 8, g.mask8() ? 1 : 4, 1).S) {
+            if (cost < best && line_cfg(t, D, 0, 1, 8, 8, 8, g.mask8() ? 1 : 4, 1).S) {
                 best = cost;
                 g.L = L; g.ty = ty; g.tz = tz;
                 g.npy = npy; g.npz = npz; g.nsteps = ns;
             }
         }
+    }
     if (best >= 1e300) return false;
     g.py = g.ty + g.ry;
     g.npad = g.py * (g.tz + g.rz);
-    for (int k = 0; k < D; k++) g.shift[k] = -dY(ord[k]) - dz[ord[k]] * g.py;
+    for (int k = 0; k < D; k++) {
+        g.shift[k] = -dY(ord[k]) - dz[ord[k]] * g.py;
+        g.back[k] = g.delta[k] * (g.npad | 1) + g.shift[k];
+    }
     // patches in ticket order: by the step they start at (dependencies start no later), then Z, Y
     std::vector<std::pair<long, int>> order;
     for (int pz = 0; pz < g.npz; pz++)
@@ -288,9 +306,6 @@ inline bool line_layout(int n, long nnz, const TileGrid &G, int sms, LineHost &h
 // its row's entry k at (patch*nsteps + step)*D*L + k*L + line.  One thread
 // per slot, so the writes coalesce; a block covers consecutive steps, so the
 // strided reads of consecutive rows of a line share cache lines.
-struct LineSlot {
-    int row;  // -1: no row
-};
 template <bool UPPER>
 __device__ __forceinline__ int line_slot_row(const LineGeo &g, const int *__restrict__ patch, long slot)
 {
@@ -409,6 +424,83 @@ __device__ __forceinline__ int line_wait(const int *p, int target, int *err, uns
     }
     return v;
 }
+// loads and stores at 32-bit shared addresses, in program order with the barriers
+template <typename T>
+__device__ __forceinline__ T lds(uint32_t a)
+{
+    if constexpr (sizeof(T) == 8) {
+        double v;
+        asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+        return v;
+    } else if constexpr (sizeof(T) == 4) {
+        uint32_t v;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+        T o;
+        memcpy(&o, &v, 4);
+        return o;
+    } else if constexpr (sizeof(T) == 2) {
+        uint16_t v;
+        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory");
+        T o;
+        memcpy(&o, &v, 2);
+        return o;
+    } else {
+        uint32_t v;
+        asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+        return (T)v;
+    }
+}
+// the same for a stage's data, which nobody writes while it is read: free to
+// move across the step barriers, but not above the wait for the stage, whose
+// addresses come from after_wait
+__device__ __forceinline__ uint32_t after_wait(uint32_t a)
+{
+    asm volatile("mov.u32 %0, %0;" : "+r"(a)::"memory");
+    return a;
+}
+template <typename T>
+__device__ __forceinline__ T lds_stage(uint32_t a)
+{
+    if constexpr (sizeof(T) == 8) {
+        double v;
+        asm("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
+        return v;
+    } else if constexpr (sizeof(T) == 4) {
+        uint32_t v;
+        asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+        T o;
+        memcpy(&o, &v, 4);
+        return o;
+    } else if constexpr (sizeof(T) == 2) {
+        uint16_t v;
+        asm("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+        T o;
+        memcpy(&o, &v, 2);
+        return o;
+    } else {
+        uint32_t v;
+        asm("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a));
+        return (T)v;
+    }
+}
+template <typename T>
+__device__ __forceinline__ void sts(uint32_t a, T v)
+{
+    if constexpr (sizeof(T) == 8) asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+    else asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void st_publish_if(bool on, double *p, double v)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.relaxed.gpu.global.f64 [%0], %1;\n\t}" ::"l"(p),
+                 "d"(v), "r"((uint32_t)on)
+                 : "memory");
+}
+__device__ __forceinline__ void st_publish_if(bool on, float *p, float v)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.relaxed.gpu.global.f32 [%0], %1;\n\t}" ::"l"(p),
+                 "f"(v), "r"((uint32_t)on)
+                 : "memory");
+}
 __device__ __forceinline__ void line_bar(int id, int count)
 {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
@@ -419,24 +511,40 @@ __device__ __forceinline__ void cp_async_mbar_arrive(uint64_t *bar)
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-template <typename VT, typename FT, typename DT, bool UPPER, int KC, int W>
-__global__ void __launch_bounds__(LINE_PATCH *KC + LINE_HELPERS + 32 * LINE_POLL_WARPS)
+// poller warps for nh halo lines of KC columns (a lane each)
+__host__ __device__ constexpr int line_poll_warps(int nh, int KC) { return nh * KC > 32 ? (nh * KC + 31) / 32 : 1; }
+__host__ __device__ constexpr int line_threads_max(int KC, int W)
+{
+    return line_patch(W) * KC + 2 * LINE_HELPERS + 32 * line_poll_warps(LINE_HALO_MAX, KC);
+}
+
+// PIVOT: instead of solving, the pivots of an ILU(0) whose eliminations only
+// reach the diagonal (see k_line_pairs): rhs and out are A's diagonal and the
+// pivots, the stream holds a_ij and a_ji of the W lower entries, and the sum
+// subtracts (a_ij / d_j) * a_ji in the order of the reference's IKJ update.
+// SU: steps unrolled (a divisor of the stage length).
+template <typename VT, typename FT, typename DT, bool UPPER, int KC, int W, bool PIVOT, int SU>
+__global__ void __launch_bounds__(line_threads_max(KC, W))
     k_trsv_lines(const __grid_constant__ LineGeo G, const __grid_constant__ LineArgs<VT, FT, DT> A)
 {
     using MK = typename std::conditional<(W == 2 || W == 3), uint8_t, uint32_t>::type;
+    static_assert(!PIVOT || (W > 0 && !UPPER), "the pivots run on the lower triangle");
+    constexpr int L = line_patch(W), T = L * KC, RS = T | 1;
     extern __shared__ __align__(128) unsigned char line_smem[];
     __shared__ __align__(8) uint64_t full[LINE_NS_MAX];
-    __shared__ int s_item, cdone, drained, hcnt[LINE_POLL_WARPS];
+    __shared__ int s_item, cdone, drained, hcnt[line_poll_warps(LINE_HALO_MAX, KC)];
     __shared__ unsigned s_half;
-    const int D = W > 0 ? W : G.D;
-    const int L = G.L, T = L * KC, S = A.S, NS = A.NS, RM = A.RL - 1, NP = A.NP;
-    const LineSmem M = LineSmem::of(G, S, NS, A.RL, KC, sizeof(VT), sizeof(FT), UPPER ? sizeof(DT) : 0, sizeof(MK));
+    const int D = W > 0 ? W : G.D, NV = PIVOT ? 2 * W : D;
+    const int S = A.S, NS = A.NS, RL = A.RL, NP = A.NP;
+    const LineSmem M = LineSmem::of(G, NV, S, NS, RL, KC, sizeof(VT), sizeof(FT), UPPER ? sizeof(DT) : 0, sizeof(MK));
     VT *ring = (VT *)(line_smem + M.ring);
     VT *s_rhs = (VT *)(line_smem + M.rhs);
     FT *s_pv = (FT *)(line_smem + M.pv);
     DT *s_dinv = (DT *)(line_smem + M.dinv);
     MK *s_mask = (MK *)(line_smem + M.mask);
-    int *s_q0 = (int *)(line_smem + M.tab), *s_off = s_q0 + L, *s_pad = s_off + L;
+    // per line: logical row of step 0 (first row - first active step), first
+    // active step (out of reach: no line), ring column
+    int4 *s_tab = (int4 *)(line_smem + M.tab);
     const int tid = threadIdx.x;
     const int PsK = M.Ps * KC;
     const int nst = G.nsteps / S;
@@ -463,7 +571,7 @@ __global__ void __launch_bounds__(LINE_PATCH *KC + LINE_HELPERS + 32 * LINE_POLL
             cdone = 0;
             drained = 0;
         }
-        if (tid < LINE_POLL_WARPS) hcnt[tid] = -G.maxd;
+        if (tid < NP) hcnt[tid] = -G.maxd;
         __syncthreads();
         const int item = s_item;
         if (item >= items) break;
@@ -471,131 +579,259 @@ __global__ void __launch_bounds__(LINE_PATCH *KC + LINE_HELPERS + 32 * LINE_POLL
         const int pY = A.patch[2 * rank], pZ = A.patch[2 * rank + 1];
         for (int l = tid; l < L; l += blockDim.x) {
             const int Yl = l % G.ty, Zl = l / G.ty;
-            s_q0[l] = G.line_q0(pY, pZ, Yl, Zl);
-            s_off[l] = G.al * Yl + G.be * Zl;
-            s_pad[l] = (Zl + G.rz) * G.py + Yl + G.ry;
+            const int q0 = G.line_q0(pY, pZ, Yl, Zl), off = G.al * Yl + G.be * Zl;
+            s_tab[l] = make_int4(q0 - off, q0 >= 0 ? off : (1 << 30), ((Zl + G.rz) * G.py + Yl + G.ry) * KC, 0);
         }
         __syncthreads();
         VT *xpub = A.xb + (s_half ? A.xb_half : 0);
         if (tid < T) {
             // ------------------------------------------------ compute
+            // One warp per scheduler runs this loop, so a step costs its
+            // instructions as much as its latencies: with the ring indexed
+            // afresh for every entry through generic pointers a 7-point step
+            // took 560 cycles, of which the sums are 40.  So every step is
+            // stored twice, RL ring rows apart, an entry is read at a
+            // constant distance from a moving row without a wrap (the row
+            // returns to the lower copy between stages: RL is a multiple of
+            // S), and all addresses are 32-bit shared ones that advance by
+            // constants.
             const int l = tid / KC, c = tid % KC;
-            const int q0 = s_q0[l], off = s_off[l];
+            const int4 tab = s_tab[l];
             const int e = __ldg(A.exp_of + l);
-            VT *pub = e >= 0 ? xpub + ((long)item * G.nsteps * G.E + e) * KC + c : nullptr;
             const long pstep = (long)G.E * KC;
-            VT *rcol = ring + s_pad[l] * KC + c;
+            VT *pub = xpub + ((long)item * G.nsteps * G.E + max(e, 0)) * KC + c;
+            const int xlo = e >= 0 ? tab.y : INT_MAX;  // published steps [xlo, xlo + nx)
+            const uint32_t rstep = (uint32_t)(PsK * sizeof(VT)), rlen = (uint32_t)RL * rstep;
+            uint32_t row = smem_u32(ring) + rlen + (uint32_t)((tab.z + c) * sizeof(VT));  // in the upper copy
+            const uint32_t row_end = row + rlen;
             int avail = -G.maxd;
             bool landed = true;
+            int slot = (int)(cnt0 % (unsigned)NS);
+            unsigned par = (cnt0 / (unsigned)NS) & 1u;
+            uint32_t back[W > 0 ? W : 1];  // ring distance of each diagonal, in bytes
+            if constexpr (W > 0) {
+#pragma unroll
+                for (int k = 0; k < W; k++) back[k] = (uint32_t)(G.back[k] * KC * (int)sizeof(VT));
+            }
+            const uint32_t a_pv = smem_u32(s_pv) + (uint32_t)(l * sizeof(FT)), a_mk = smem_u32(s_mask) + (uint32_t)(l * sizeof(MK));
+            const uint32_t a_dv = smem_u32(s_dinv) + (uint32_t)(l * sizeof(DT)), a_rh = smem_u32(s_rhs) + (uint32_t)(tid * sizeof(VT));
+            int tau = 0;
             for (int g = 0; g < nst; g++) {
-                const unsigned st = cnt0 + (unsigned)g;
-                const int slot = (int)(st % (unsigned)NS);
-                if (landed) landed = mbar_wait_bounded(&full[slot], (st / (unsigned)NS) & 1u, A.err);
-                line_wait(&drained, (g + 1) * S - A.RL, A.err, 0);
-                const FT *pv = s_pv + (size_t)slot * S * D * L + l;
-                const MK *mk = s_mask + (size_t)slot * S * L + l;
-                const DT *dv = s_dinv + (size_t)slot * S * L + l;
-                const VT *rh = s_rhs + (size_t)slot * S * M.RS + tid;
-                for (int s = 0; s < S; s++) {
-                    const int tau = g * S + s, x = tau - off;
-                    VT acc = rh[s * M.RS];
-                    const uint32_t m = mk[s * L];
-                    if (UPPER) acc = (VT)(acc * (VT)dv[s * L]);
-                    const FT *pvs = pv + (size_t)s * D * L;
-                    FT v[W > 0 ? W : 1];
+                if (landed) landed = mbar_wait_bounded(&full[slot], par, A.err);
+                line_wait(&drained, (g + 1) * S - RL, A.err, 0);
+                const uint32_t first = (uint32_t)(slot * S);
+                uint32_t pv = after_wait(a_pv + first * (uint32_t)(NV * L * sizeof(FT)));
+                uint32_t mk = after_wait(a_mk + first * (uint32_t)(L * sizeof(MK)));
+                uint32_t dv = after_wait(a_dv + first * (uint32_t)(L * sizeof(DT)));
+                uint32_t rh = after_wait(a_rh + first * (uint32_t)(RS * sizeof(VT)));
+                // a step's own data is loaded during the step before it
+                VT rr[2], dd[2];
+                uint32_t mm[2];
+                constexpr int NVC = W > 0 ? (PIVOT ? 2 * W : W) : 1;
+                FT vv[2][NVC];
+                auto fetch = [&](int b, uint32_t u) {
+                    rr[b] = lds_stage<VT>(rh + u * (uint32_t)(RS * sizeof(VT)));
+                    mm[b] = lds_stage<MK>(mk + u * (uint32_t)(L * sizeof(MK)));
+                    if constexpr (UPPER) dd[b] = (VT)lds_stage<DT>(dv + u * (uint32_t)(L * sizeof(DT)));
                     if constexpr (W > 0) {
 #pragma unroll
-                        for (int k = 0; k < W; k++) v[k] = pvs[k * L];
+                        for (int k = 0; k < NVC; k++)
+                            vv[b][k] = lds_stage<FT>(pv + (u * (uint32_t)NVC + (uint32_t)k) * (uint32_t)(L * sizeof(FT)));
                     }
-                    // the halo values this step may read (steps before it)
-                    if (avail < tau) {
-                        avail = line_wait(&hcnt[0], tau, A.err, 0);
-                        for (int w = 1; w < NP; w++) avail = min(avail, line_wait(&hcnt[w], tau, A.err, 0));
-                    }
-                    if (q0 >= 0 && (unsigned)x < (unsigned)G.nx) {
+                };
+                fetch(0, 0);
+                for (int s = 0; s < S; s += SU) {
+#pragma unroll
+                    for (int u = 0; u < SU; u++) {
+                        const int cb = SU > 1 ? (u & 1) : 0, nb = cb ^ 1;
+                        // the halo values this step may read (steps before it)
+                        if (avail < tau) {
+                            avail = line_wait(&hcnt[0], tau, A.err, 0);
+                            for (int w = 1; w < NP; w++) avail = min(avail, line_wait(&hcnt[w], tau, A.err, 0));
+                        }
+                        VT acc;
                         if constexpr (W > 0) {
+                            VT y[W];
+#pragma unroll
+                            for (int k = 0; k < W; k++) y[k] = lds<VT>(row - back[k]);
+                            if (u + 1 < SU || s + SU < S) fetch(nb, (uint32_t)(u + 1));
+                            acc = rr[cb];
+                            if constexpr (UPPER) acc = (VT)(acc * dd[cb]);
 #pragma unroll
                             for (int k = 0; k < W; k++) {
-                                const VT y = rcol[((tau - G.delta[k]) & RM) * PsK - G.shift[k] * KC];
-                                const VT a2 = msub(acc, y, (VT)FVal<FT>::cvt(v[k]));
-                                acc = (m >> k) & 1u ? a2 : acc;
+                                if constexpr (PIVOT) {
+                                    const VT q = vv[cb][k] / y[k];
+                                    const VT t = q * vv[cb][W + k];
+                                    if ((mm[cb] >> k) & 1u) acc = acc - t;
+                                } else {
+                                    const VT t = msub(acc, y[k], (VT)FVal<FT>::cvt(vv[cb][k]));
+                                    if ((mm[cb] >> k) & 1u) acc = t;
+                                }
+                            }
+                            if constexpr (PIVOT) {
+                                if (fabs(acc) < 1e-20) acc = 1e-20;
                             }
                         } else {
+                            // chunks of 8 entries, the next chunk's loads before
+                            // this one's sum (k is a constant in every copy)
+                            VT y[2][8];
+                            FT e8[2][8];
+                            auto chunk = [&](auto kb_, int b) {
+                                constexpr int kb = decltype(kb_)::value;
+#pragma unroll
+                                for (int j = 0; j < 8; j++) {
+                                    const int k = kb + j, kk = k < D ? k : 0;
+                                    y[b][j] = lds<VT>(row - (uint32_t)(G.back[k] * KC * (int)sizeof(VT)));
+                                    e8[b][j] = lds_stage<FT>(pv + (uint32_t)(kk * L * sizeof(FT)));
+                                }
+                            };
+                            const uint32_t m = mm[cb];
+                            auto sum = [&](auto kb_, int b) {
+                                constexpr int kb = decltype(kb_)::value;
+#pragma unroll
+                                for (int j = 0; j < 8; j++) {
+                                    const VT t = msub(acc, y[b][j], (VT)FVal<FT>::cvt(e8[b][j]));
+                                    if ((m >> (kb + j)) & 1u) acc = t;
+                                }
+                            };
+                            using std::integral_constant;
+                            chunk(integral_constant<int, 0>(), 0);
+                            acc = rr[cb];
+                            if constexpr (UPPER) acc = (VT)(acc * dd[cb]);
+                            if (D > 8) chunk(integral_constant<int, 8>(), 1);
+                            sum(integral_constant<int, 0>(), 0);
+                            if (D > 8) {
+                                if (D > 16) chunk(integral_constant<int, 16>(), 0);
+                                sum(integral_constant<int, 8>(), 1);
+                                if (D > 16) {
+                                    if (D > 24) chunk(integral_constant<int, 24>(), 1);
+                                    sum(integral_constant<int, 16>(), 0);
+                                    if (D > 24) sum(integral_constant<int, 24>(), 1);
+                                }
+                            }
+                            if (s + SU < S) fetch(nb, 1);
+                        }
+                        // a step outside the line is stored too: no entry names it
+                        sts<VT>(row, acc);
+                        sts<VT>(row - rlen, acc);
+                        st_publish_if((unsigned)(tau - xlo) < (unsigned)G.nx, pub, acc);
+                        pub += pstep;
+                        row += rstep;
+                        tau++;
+                        if constexpr (SU == 1) {
+                            rr[0] = rr[1];
+                            mm[0] = mm[1];
+                            if constexpr (UPPER) dd[0] = dd[1];
+#pragma unroll
+                            for (int k = 0; k < NVC; k++) vv[0][k] = vv[1][k];
+                        }
+                        line_bar(1, T);
+                    }
+                    rh += (uint32_t)(SU * RS * sizeof(VT));
+                    mk += (uint32_t)(SU * L * sizeof(MK));
+                    if (UPPER) dv += (uint32_t)(SU * L * sizeof(DT));
+                    pv += (uint32_t)(SU * NV * L * sizeof(FT));
+                }
+                if (row == row_end) row -= rlen;
+                if (tid == 0) st_release_cta(&cdone, tau);
+                if (++slot == NS) {
+                    slot = 0;
+                    par ^= 1u;
+                }
+            }
+        } else if (tid < T + 2 * LINE_HELPERS) {
+            // ------------------------------------------------ staging, draining
+            const bool drain = tid >= T + LINE_HELPERS;
+            const int h = tid - T - (drain ? LINE_HELPERS : 0);
+            const long base = (long)rank * G.nsteps;
+            const int lg = 31 - __clz(S);  // S is a power of two
+            const int nel = T * S;
+            // element i of a stage: column i % KC, step i / KC % S, line i / KC / S
+            auto element = [&](int i, int tau0, int &l, int &s, int &c, long &o) {
+                c = i % KC;
+                s = (i / KC) & (S - 1);
+                l = (i / KC) >> lg;
+                const int4 t = s_tab[l];
+                const int tau = tau0 + s, col = grp * KC + c;
+                const int q = t.x + tau;
+                const int row = UPPER ? G.n - 1 - q : q;
+                o = KC == 1 ? (long)row : (long)row * A.k + col;
+                const bool in = (unsigned)(tau - t.y) < (unsigned)G.nx && (KC == 1 || col < A.k);
+                return in ? t.z + c : -1;  // ring column
+            };
+            if (!drain) {
+                auto stage = [&](int g) {
+                    const unsigned st = cnt0 + (unsigned)g;
+                    const int slot = (int)(st % (unsigned)NS);
+                    if (h == 0) {
+                        const uint32_t bv = (uint32_t)(S * NV * L * sizeof(FT)), bm = (uint32_t)(S * L * sizeof(MK));
+                        const uint32_t bd = UPPER ? (uint32_t)(S * L * sizeof(DT)) : 0u;
+                        mbar_expect_tx(&full[slot], bv + bm + bd);
+                        bulk_g2s(s_pv + (size_t)slot * S * NV * L, A.pv + (base + (long)g * S) * NV * L, bv, &full[slot]);
+                        bulk_g2s(s_mask + (size_t)slot * S * L, (const MK *)A.mask + (base + (long)g * S) * L, bm,
+                                 &full[slot]);
+                        if (UPPER)
+                            bulk_g2s(s_dinv + (size_t)slot * S * L, A.dinv + (base + (long)g * S) * L, bd, &full[slot]);
+                    }
+                    VT *rb = s_rhs + (size_t)slot * S * RS;
 #pragma unroll 4
-                            for (int k = 0; k < D; k++) {
-                                const VT y = rcol[((tau - G.delta[k]) & RM) * PsK - G.shift[k] * KC];
-                                const VT a2 = msub(acc, y, (VT)FVal<FT>::cvt(pvs[k * L]));
-                                acc = (m >> k) & 1u ? a2 : acc;
+                    for (int i = h; i < nel; i += LINE_HELPERS) {
+                        int l, s, c;
+                        long o;
+                        if (element(i, g * S, l, s, c, o) >= 0)
+                            cp_async_n<sizeof(VT)>(rb + s * RS + l * KC + c, A.rhs + o);
+                    }
+                    cp_async_mbar_arrive(&full[slot]);
+                };
+                for (int g = 0; g < NS && g < nst; g++) stage(g);
+                for (int g = NS; g < nst; g++) {
+                    line_wait(&cdone, (g - NS + 1) * S, A.err, 100);
+                    stage(g);
+                }
+            } else {
+                // re-arm this patch's part of the other half for the next launch
+                VT *xr = A.xb + (s_half ? 0 : A.xb_half) + (long)item * G.nsteps * G.E * KC;
+                for (int i = h; i < G.nsteps * G.E * KC; i += LINE_HELPERS) xr[i] = Sentinel<VT>::value();
+                for (int g = 0; g < nst; g++) {
+                    line_wait(&cdone, (g + 1) * S, A.err, 200);
+                    for (int i0 = h; i0 < nel; i0 += 4 * LINE_HELPERS) {
+                        VT v[4];
+                        long o[4];
+#pragma unroll
+                        for (int u = 0; u < 4; u++) {
+                            const int i = i0 + u * LINE_HELPERS;
+                            o[u] = -1;
+                            if (i < nel) {
+                                int l, s, c;
+                                long a;
+                                const int rc = element(i, g * S, l, s, c, a);
+                                if (rc >= 0) {
+                                    v[u] = ring[((g * S + s) & (RL - 1)) * PsK + rc];
+                                    o[u] = a;
+                                }
                             }
                         }
-                        rcol[(tau & RM) * PsK] = acc;
-                        if (pub) st_publish(pub + tau * pstep, acc);
-                    }
-                    line_bar(1, T);
-                }
-                if (tid == 0) st_release_cta(&cdone, (g + 1) * S);
-            }
-        } else if (tid < T + LINE_HELPERS) {
-            // ------------------------------------------------ staging and draining
-            const int h = tid - T;
-            const long base = (long)rank * G.nsteps;
-            const int per = S * KC;
-            const int nel = L * per;
-            auto stage = [&](int g) {
-                const unsigned st = cnt0 + (unsigned)g;
-                const int slot = (int)(st % (unsigned)NS);
-                if (h == 0) {
-                    const uint32_t bv = (uint32_t)(S * D * L * sizeof(FT)), bm = (uint32_t)(S * L * sizeof(MK));
-                    const uint32_t bd = UPPER ? (uint32_t)(S * L * sizeof(DT)) : 0u;
-                    mbar_expect_tx(&full[slot], bv + bm + bd);
-                    bulk_g2s(s_pv + (size_t)slot * S * D * L, A.pv + (base + (long)g * S) * D * L, bv, &full[slot]);
-                    bulk_g2s(s_mask + (size_t)slot * S * L, (const MK *)A.mask + (base + (long)g * S) * L, bm, &full[slot]);
-                    if (UPPER)
-                        bulk_g2s(s_dinv + (size_t)slot * S * L, A.dinv + (base + (long)g * S) * L, bd, &full[slot]);
-                }
-                VT *rb = s_rhs + (size_t)slot * S * M.RS;
-                for (int i = h; i < nel; i += LINE_HELPERS) {
-                    const int l = i / per, r = i % per, s = r / KC, c = r % KC;
-                    const int q0 = s_q0[l], x = g * S + s - s_off[l], col = grp * KC + c;
-                    if (q0 >= 0 && (unsigned)x < (unsigned)G.nx && (KC == 1 || col < A.k)) {
-                        const long row = UPPER ? G.n - 1 - (q0 + x) : q0 + x;
-                        cp_async_n<sizeof(VT)>(rb + s * M.RS + l * KC + c, A.rhs + (KC == 1 ? row : row * A.k + col));
-                    }
-                }
-                cp_async_mbar_arrive(&full[slot]);
-            };
-            for (int g = 0; g < NS && g < nst; g++) stage(g);
-            for (int g = 0; g < nst; g++) {
-                line_wait(&cdone, (g + 1) * S, A.err, 40);
-                if (g + NS < nst) stage(g + NS);
-                for (int i = h; i < nel; i += LINE_HELPERS) {
-                    const int l = i / per, r = i % per, s = r / KC, c = r % KC;
-                    const int q0 = s_q0[l], tau = g * S + s, x = tau - s_off[l], col = grp * KC + c;
-                    if (q0 >= 0 && (unsigned)x < (unsigned)G.nx && (KC == 1 || col < A.k)) {
-                        const long row = UPPER ? G.n - 1 - (q0 + x) : q0 + x;
-                        const long o = KC == 1 ? row : row * A.k + col;
-                        A.out[o] = ring[(tau & RM) * PsK + s_pad[l] * KC + c];
-                        if (A.reset_other) A.reset_other[o] = Sentinel<VT>::value();
-                    }
-                }
-                line_bar(2, LINE_HELPERS);
-                if (h == 0) st_release_cta(&drained, (g + 1) * S);
-            }
-            // re-arm this patch's part of the other half for the next launch
-            VT *xr = A.xb + (s_half ? 0 : A.xb_half) + (long)item * G.nsteps * G.E * KC;
-            for (int i = h; i < G.nsteps * G.E * KC; i += LINE_HELPERS) xr[i] = Sentinel<VT>::value();
-        } else if ((tid - T - LINE_HELPERS) / 32 < NP) {
-            // ------------------------------------------------ halo
-            const int pw = (tid - T - LINE_HELPERS) / 32, lane = tid & 31;
-            const VT *src[LINE_ITEMS];
-            int x0[LINE_ITEMS], x1[LINE_ITEMS], pos[LINE_ITEMS], rc[LINE_ITEMS];
-            const long pstep = (long)G.E * KC;
 #pragma unroll
-            for (int j = 0; j < LINE_ITEMS; j++) {
-                const int i = (j * NP + pw) * 32 + lane;
-                src[j] = nullptr;
-                x0[j] = x1[j] = rc[j] = 0;
-                pos[j] = -G.maxd;
+                        for (int u = 0; u < 4; u++)
+                            if (o[u] >= 0) {
+                                A.out[o[u]] = v[u];
+                                if (A.reset_other) A.reset_other[o[u]] = Sentinel<VT>::value();
+                            }
+                    }
+                    line_bar(2, LINE_HELPERS);
+                    if (h == 0) st_release_cta(&drained, (g + 1) * S);
+                }
+            }
+        } else {
+            // ------------------------------------------------ halo
+            // each lane follows one halo line (a column of it): pos is the
+            // first step whose value it does not have yet
+            const int pw = (tid - T - 2 * LINE_HELPERS) / 32, lane = tid & 31;
+            const VT *src = nullptr;  // the value of step pos
+            int x1 = 0, pos = INT_MAX, rc = 0;
+            const long pstep = (long)G.E * KC;
+            {
+                const int i = pw * 32 + lane;
                 if (i < G.nh * KC) {
                     const int hl = i / KC, c = i % KC;
                     const int Yl = __ldg(A.halo + 2 * hl), Zl = __ldg(A.halo + 2 * hl + 1);
@@ -605,11 +841,11 @@ __global__ void __launch_bounds__(LINE_PATCH *KC + LINE_HELPERS + 32 * LINE_POLL
                         const int ro = __ldg(A.rank_of + (pZ + dpZ) * G.npy + pY + dpY);
                         const int off_o = G.al * Yo + G.be * Zo, off_h = G.al * Yl + G.be * Zl;
                         const int eo = __ldg(A.exp_of + Zo * G.ty + Yo);
-                        // value of step t here: step t + (off_o - off_h) of the owner
-                        src[j] = xpub + (((long)ro * A.ngroups + grp) * G.nsteps + (off_o - off_h)) * pstep + eo * KC + c;
-                        x0[j] = off_h;  // active steps [x0, x1)
-                        x1[j] = off_h + G.nx;
-                        rc[j] = ((Zl + G.rz) * G.py + Yl + G.ry) * KC + c;
+                        // active steps [off_h, off_h + nx) here are [off_o, off_o + nx) of the owner
+                        src = xpub + (((long)ro * A.ngroups + grp) * G.nsteps + off_o) * pstep + eo * KC + c;
+                        pos = off_h;
+                        x1 = off_h + G.nx;
+                        rc = ((Zl + G.rz) * G.py + Yl + G.ry) * KC + c;
                     }
                 }
             }
@@ -619,29 +855,32 @@ __global__ void __launch_bounds__(LINE_PATCH *KC + LINE_HELPERS + 32 * LINE_POLL
             unsigned long long t0 = 0;
             long spins = 0;
             while (published < G.nsteps) {
-                const int lim = min(ld_acquire_cta(&cdone) + A.RL - G.maxd, G.nsteps);
-                int mn = lim;
-#pragma unroll
-                for (int j = 0; j < LINE_ITEMS; j++) {
-                    if (!src[j] || !ok) continue;
-                    const int p = pos[j], m = min(lim - p, LINE_WINDOW);
+                const int lim = min(ld_acquire_cta(&cdone) + RL - G.maxd, G.nsteps);
+                const int m = min(min(lim, x1) - pos, LINE_WINDOW);  // values this lane may take now
+                if (m > 0 && ok) {
                     VT v[LINE_WINDOW];
+                    const VT *q = src;
 #pragma unroll
                     for (int u = 0; u < LINE_WINDOW; u++) {
-                        v[u] = (VT)0;
-                        if (u < m && p + u >= x0[j] && p + u < x1[j]) v[u] = ld_poll(src[j] + (p + u) * pstep);
+                        v[u] = Sentinel<VT>::value();
+                        if (u < m) v[u] = ld_poll(q);
+                        q += pstep;
                     }
                     int r = 0;
 #pragma unroll
-                    for (int u = 0; u < LINE_WINDOW; u++) {
-                        if (r == u && u < m && !Sentinel<VT>::is(v[u])) {
-                            if (p + u >= x0[j] && p + u < x1[j]) ring[((p + u) & RM) * PsK + rc[j]] = v[u];
-                            r = u + 1;
+                    for (int u = 0; u < LINE_WINDOW; u++)
+                        if (r == u && !Sentinel<VT>::is(v[u])) r = u + 1;
+#pragma unroll
+                    for (int u = 0; u < LINE_WINDOW; u++)
+                        if (u < r) {
+                            VT *w = ring + ((pos + u) & (RL - 1)) * PsK + rc;
+                            w[0] = v[u];
+                            w[RL * PsK] = v[u];
                         }
-                    }
-                    pos[j] = p + r;
-                    mn = min(mn, p + r);
+                    pos += r;
+                    src += r * pstep;
                 }
+                int mn = pos < x1 && ok ? min(pos, lim) : lim;
                 if (brk && ok) mn = min(mn, 0);
                 mn = __reduce_min_sync(0xffffffffu, mn);
                 if (mn > published) {
@@ -652,7 +891,7 @@ __global__ void __launch_bounds__(LINE_PATCH *KC + LINE_HELPERS + 32 * LINE_POLL
                     spins = 0;
                 } else if (mn >= lim) {
                     // the ring is full: the compute threads are behind (their waits are bounded)
-                    line_wait(&cdone, lim + G.maxd - A.RL + 1, A.err, 64);
+                    line_wait(&cdone, lim + G.maxd - RL + 1, A.err, 40);
                     t0 = 0;
                 } else if ((++spins & 63) == 0) {
                     const unsigned long long now = gtimer();
@@ -676,7 +915,7 @@ __global__ void __launch_bounds__(LINE_PATCH *KC + LINE_HELPERS + 32 * LINE_POLL
 inline int line_kc(const LineGeo &g, int k)
 {
     for (int kc = k >= 3 ? 4 : k; kc > 1; kc = kc == 4 ? 2 : 1)
-        if (line_cfg(g, 0, kc, sizeof(double), sizeof(double), sizeof(double), g.mask8() ? 1 : 4, 1).S) return kc;
+        if (line_cfg(g, g.D, 0, kc, sizeof(double), sizeof(double), sizeof(double), g.mask8() ? 1 : 4, 1).S) return kc;
     return 1;
 }
 
@@ -700,27 +939,29 @@ inline void line_xchg_rearm(LineXchg<VT> &X, cudaStream_t s)
     XS_CUDA(cudaMemsetAsync(X.ctl.p, 0, sizeof(unsigned), s));
 }
 
-template <typename VT, typename FT, typename DT, bool UPPER, int KC>
-inline void launch_trsv_lines(const LinePlan &P, const FT *pv, const DT *dinv, LineXchg<VT> &X, int k, const VT *rhs,
-                              VT *out, VT *reset_other, const int *done_flag, int *err, cudaStream_t s)
+template <typename VT, typename FT, typename DT, bool UPPER, int KC, bool PIVOT = false>
+inline void launch_trsv_lines(const LinePlan &P, const FT *pv, const uint8_t *mask8, const DT *dinv, LineXchg<VT> &X,
+                              int k, const VT *rhs, VT *out, VT *reset_other, const int *done_flag, int *err,
+                              cudaStream_t s)
 {
     const LineGeo &g = P.g;
     const int ng = (k + KC - 1) / KC, items = g.npatch * ng, sms = geom().sms;
     const bool m8 = g.mask8();
-    const LineCfg c = line_cfg(g, items, KC, sizeof(VT), sizeof(FT), UPPER ? sizeof(DT) : 0, m8 ? 1 : 4, sms);
+    const LineCfg c = line_cfg(g, PIVOT ? 2 * g.D : g.D, items, KC, sizeof(VT), sizeof(FT), UPPER ? sizeof(DT) : 0,
+                               m8 ? 1 : 4, sms);
     if (c.S == 0 || !X.x.p || X.half != (size_t)items * g.nsteps * g.E * KC) throw Status(XS_ERR_ORDER);
     LineArgs<VT, FT, DT> A;
     A.patch = P.patch.p; A.rank_of = P.rank_of.p; A.halo = P.halo.p; A.exp_of = P.exp_of.p;
     A.pv = pv;
-    A.mask = m8 ? (const void *)P.mask8.p : (const void *)P.mask32.p;
+    A.mask = m8 ? (const void *)mask8 : (const void *)P.mask32.p;
     A.dinv = dinv;
     A.xb = X.x.p; A.xb_half = (long)X.half; A.ctl = X.ctl.p;
     A.S = c.S; A.NS = c.NS; A.RL = c.RL;
-    A.NP = std::max(1, std::min(LINE_POLL_WARPS, (g.nh * KC + 31) / 32));
+    A.NP = line_poll_warps(g.nh, KC);
     A.k = k; A.ngroups = ng;
     A.rhs = rhs; A.out = out; A.reset_other = reset_other;
-    A.done_flag = done_flag; A.err = err; A.brk = P.brk;
-    const int threads = g.L * KC + LINE_HELPERS + 32 * A.NP;
+    A.done_flag = done_flag; A.err = err; A.brk = PIVOT ? -1 : P.brk;
+    const int threads = line_patch(g.D) * KC + 2 * LINE_HELPERS + 32 * A.NP;
     const int per_sm = c.smem <= 112 * 1024 && 2 * threads <= 2048 ? 2 : 1;
     const int grid = std::min(items, sms * per_sm);
     auto go = [&](auto kern) {
@@ -728,9 +969,92 @@ inline void launch_trsv_lines(const LinePlan &P, const FT *pv, const DT *dinv, L
         XS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LINE_SMEM_MAX));
         launch_pdl(kern, dim3(grid), dim3(threads), c.smem, s, g, A);
     };
-    if (g.D == 3) go(k_trsv_lines<VT, FT, DT, UPPER, KC, 3>);
-    else if (g.D == 2) go(k_trsv_lines<VT, FT, DT, UPPER, KC, 2>);
-    else go(k_trsv_lines<VT, FT, DT, UPPER, KC, 0>);
+    // unrolled steps: 2 and 4 measured alike, 8 slower (instruction cache), 1
+    // slower by a sixth (LU solve 128^3 7-point: 319, 318, 330 and 362 us)
+    constexpr int SU = 4;
+    const bool unrolled = c.S % SU == 0;
+    if (g.D == 3 && unrolled) go(k_trsv_lines<VT, FT, DT, UPPER, KC, 3, PIVOT, SU>);
+    else if (g.D == 3) go(k_trsv_lines<VT, FT, DT, UPPER, KC, 3, PIVOT, 1>);
+    else if (g.D == 2 && unrolled) go(k_trsv_lines<VT, FT, DT, UPPER, KC, 2, PIVOT, SU>);
+    else if (g.D == 2) go(k_trsv_lines<VT, FT, DT, UPPER, KC, 2, PIVOT, 1>);
+    else if constexpr (PIVOT) throw Status(XS_ERR_UNSUPPORTED);
+    else if (g.D == 13 && c.S % 2 == 0) go(k_trsv_lines<VT, FT, DT, UPPER, KC, 13, false, 2>);
+    else go(k_trsv_lines<VT, FT, DT, UPPER, KC, 0, false, 1>);
+}
+
+// ---------------------------------------------------------------- ILU(0) on the line schedule
+// When the sum of a lower and an upper diagonal of A is the main diagonal or
+// no diagonal at all (5- and 7-point stencils), an elimination of ILU(0)
+// changes nothing but the pivot: u_ij = a_ij, l_ij = a_ij / d_j, and
+//     d_i = a_ii - sum_j (a_ij / d_j) * a_ji,
+// a recurrence over L's dependencies with one value per row.  It runs on the
+// line schedule of the L solve (k_trsv_lines<PIVOT>), with the operations of
+// the reference's ilu0_simple in its order, so the factors are bitwise the
+// same; the rest of the factor is one elementwise pass (k_line_ilu_finish).
+// The lane-group kernel pays a cross-SM hand-off per dependency level: 4.6 ms
+// at 128^3 7-point.
+inline bool line_ilu_ok(const LinePlan &L, const LinePlan &U)
+{
+    const LineGeo &a = L.g, &b = U.g;
+    if (!a.mask8()) return false;
+    auto has = [&](int off) {
+        for (int k = 0; k < a.D; k++)
+            if (a.offq[k] == off) return true;
+        for (int k = 0; k < b.D; k++)
+            if (-b.offq[k] == off) return true;
+        return false;
+    };
+    for (int j = 0; j < a.D; j++)
+        for (int m = 0; m < b.D; m++) {
+            const int s = a.offq[j] - b.offq[m];  // lower + upper (U's offsets are logical: reversed)
+            if (s != 0 && has(s)) return false;
+        }
+    return line_cfg(a, 2 * a.D, 0, 1, 8, 8, 0, 1, 1).S != 0;
+}
+
+// the stream of the pivots: per slot a_ij and a_ji of each lower diagonal,
+// and the mask of the ones that have both (rp/ci/v: A; uptr: its diagonal)
+static __global__ void k_line_pairs(LineGeo g, const int *__restrict__ patch, const int *__restrict__ rp,
+                                    const int *__restrict__ ci, const int *__restrict__ uptr,
+                                    const double *__restrict__ v, double *__restrict__ pv, uint8_t *__restrict__ mask)
+{
+    const long m = g.slots();
+    for (long s = blockIdx.x * (long)blockDim.x + threadIdx.x; s < m; s += (long)gridDim.x * blockDim.x) {
+        const int r = line_slot_row<false>(g, patch, s);
+        double *o = pv + s / g.L * (2 * g.D) * g.L + s % g.L;
+        uint32_t b = 0;
+        int e = r >= 0 ? rp[r] : 0;
+        const int e1 = r >= 0 ? uptr[r] : 0;
+        for (int k = 0; k < g.D; k++) {
+            double a = 0.0, t = 0.0;
+            if (e < e1 && ci[e] - r == g.offq[k]) {
+                const int c = ci[e];
+                a = v[e++];
+                for (int q = uptr[c] + 1; q < rp[c + 1]; q++)
+                    if (ci[q] == r) {
+                        t = v[q];
+                        b |= 1u << k;
+                    }
+            }
+            o[(long)k * g.L] = a;
+            o[(long)(g.D + k) * g.L] = t;
+        }
+        mask[s] = (uint8_t)b;
+    }
+}
+static __global__ void k_line_diag(int n, const int *__restrict__ uptr, const double *__restrict__ v, double *d)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) d[i] = v[uptr[i]];
+}
+// luv (A's values): l_ij = a_ij / d_j, the pivots on the diagonal, U unchanged
+static __global__ void k_line_ilu_finish(int n, const int *__restrict__ rp, const int *__restrict__ ci,
+                                         const int *__restrict__ uptr, const double *__restrict__ d, double *luv)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int up = uptr[i];
+        for (int e = rp[i]; e < up; e++) luv[e] = luv[e] / __ldg(d + ci[e]);
+        luv[up] = __ldg(d + i);
+    }
 }
 
 }  // namespace xs

@@ -25,6 +25,7 @@ namespace xs {
 
 constexpr int BATCH_MAX = 16;
 constexpr int BATCH_THREADS = 256;
+constexpr int BATCH_CTAS = 4;  // resident per SM (64 registers: the loads a thread keeps in flight)
 
 // batched kernels on (1, default) or the right-hand sides solved one by one (0)
 struct BatchTuning {
@@ -51,6 +52,7 @@ __device__ bool block_reduce_cols(const double (&v)[NV], int k, RedSlot slot, do
 #pragma unroll
         for (int a = 0; a < NV; a++) {
             double s = 0.0;
+#pragma unroll 8
             for (int q = t; q < nb; q += k) s += sv[a][q];
             slot.part[((long)a * k + t) * G + blockIdx.x] = s;
         }
@@ -69,6 +71,7 @@ __device__ bool block_reduce_cols(const double (&v)[NV], int k, RedSlot slot, do
 #pragma unroll
     for (int a = 0; a < NV; a++) {
         s[a] = 0.0;
+#pragma unroll 8
         for (int b = j; b < G; b += per) s[a] += __ldcg(slot.part + ((long)a * k + c) * G + b);
     }
     __syncthreads();
@@ -79,6 +82,7 @@ __device__ bool block_reduce_cols(const double (&v)[NV], int k, RedSlot slot, do
 #pragma unroll
         for (int a = 0; a < NV; a++) {
             double acc = 0.0;
+#pragma unroll 8
             for (int q = t; q < per * k; q += k) acc += sv[a][q];
             tot[a * k + t] = acc;
         }
@@ -90,6 +94,12 @@ __device__ bool block_reduce_cols(const double (&v)[NV], int k, RedSlot slot, do
 
 inline int batch_block(int k) { return (BATCH_THREADS / k) * k; }
 inline int batch_grid() { return geom().red_grid; }
+// CTAs for n rows of k columns: one wave, fewer for small systems
+inline int batch_grid_for(int n, int k)
+{
+    const long need = ((long)n * k + batch_block(k) - 1) / batch_block(k);
+    return (int)std::max(1L, std::min<long>(std::min(batch_grid(), BATCH_CTAS * geom().sms), need));
+}
 
 // every column's solve has ended: the later kernels of the iteration skip
 __device__ inline void batch_set_all_done(const KState *st, int k, int *all_done)
@@ -105,8 +115,14 @@ enum BSpmvMode { BS_RESID = 1, BS_DOT_SIGMA = 2 };
 // MODE BS_RESID: Y = B - A X, per column r.r into sc[S_RES0SQ] (every column)
 // MODE BS_DOT_SIGMA: Y = A X, per column w.y -> sigma, alpha = tao/(sigma + small)
 //   (EpiDot1 with M_CGM_SIGMA), columns already converged skipped
-template <int MODE>
-__global__ void __launch_bounds__(BATCH_THREADS) k_bspmv(int n, int k, const int *__restrict__ rp,
+constexpr int BSPMV_CHUNK = 8;  // entries of a row loaded at once
+// KV neighbouring columns per thread (2 where k is even: the row's columns
+// and values are then read by half as many threads, and x and y as 16-byte
+// vectors): the load instructions are what bounds this kernel.  (One entry
+// of one column at a time, the form before, took 91 us per product of eight
+// columns at 96^3, two thirds of the time waiting for a row's next entry.)
+template <int MODE, int KV>
+__global__ void __launch_bounds__(BATCH_THREADS, BATCH_CTAS) k_bspmv(int n, int k, const int *__restrict__ rp,
                                                         const int *__restrict__ ci, const double *__restrict__ v,
                                                         const double *__restrict__ X, double *__restrict__ Y,
                                                         const double *__restrict__ W, KState *st, int *all_done,
@@ -114,29 +130,66 @@ __global__ void __launch_bounds__(BATCH_THREADS) k_bspmv(int n, int k, const int
 {
     __shared__ double tot[BATCH_MAX];
     if (*all_done) return;
-    const int c = threadIdx.x % k;
-    const bool active = MODE == BS_RESID || st[c].done == 0;
-    const long m = (long)n * k;
-    double acc[1] = {0.0};
-    if (active) {
-        for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < m; q += (long)gridDim.x * blockDim.x) {
-            const int i = (int)(q / k);
-            double sum = 0.0;
-            for (int e = __ldg(rp + i); e < __ldg(rp + i + 1); e++) sum += __ldg(v + e) * __ldg(X + (long)__ldg(ci + e) * k + c);
-            if (MODE == BS_RESID) {
-                const double y = __ldg(W + q) - sum;  // W = B
-                Y[q] = y;
-                acc[0] += y * y;
-            } else {
-                Y[q] = sum;
-                acc[0] += __ldg(W + q) * sum;  // W = P
+    const int kt = k / KV;  // threads per row
+    const int c = threadIdx.x % kt * KV;
+    bool active[KV], any = false;
+#pragma unroll
+    for (int u = 0; u < KV; u++) {
+        active[u] = MODE == BS_RESID || st[c + u].done == 0;
+        any |= active[u];
+    }
+    auto ldv = [](const double *p, double (&o)[KV]) {
+        if constexpr (KV == 2) {
+            const double2 d = __ldg((const double2 *)p);
+            o[0] = d.x;
+            o[1] = d.y;
+        } else {
+            o[0] = __ldg(p);
+        }
+    };
+    double acc[KV] = {};
+    if (any) {
+        // the grid stride is a multiple of k: a thread stays on its columns
+        const int step = (int)((long)gridDim.x * blockDim.x / kt);
+        for (int i = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) / kt); i < n; i += step) {
+            const long q = (long)i * k + c;
+            const int e1 = __ldg(rp + i + 1);
+            double w[KV], sum[KV] = {};
+            ldv(W + q, w);  // W = B or P
+            // a chunk's columns and values, then its gathers, then its sum:
+            // three latencies a chunk instead of one per entry
+            for (int e = __ldg(rp + i); e < e1; e += BSPMV_CHUNK) {
+                int cc[BSPMV_CHUNK];
+                double vv[BSPMV_CHUNK], xx[BSPMV_CHUNK][KV];
+#pragma unroll
+                for (int j = 0; j < BSPMV_CHUNK; j++) {
+                    const bool in = e + j < e1;
+                    cc[j] = in ? __ldg(ci + e + j) : i;
+                    vv[j] = in ? __ldg(v + e + j) : 0.0;
+                }
+#pragma unroll
+                for (int j = 0; j < BSPMV_CHUNK; j++) ldv(X + (long)cc[j] * k + c, xx[j]);
+#pragma unroll
+                for (int j = 0; j < BSPMV_CHUNK; j++)
+                    if (e + j < e1) {
+#pragma unroll
+                        for (int u = 0; u < KV; u++) sum[u] += vv[j] * xx[j][u];
+                    }
             }
+#pragma unroll
+            for (int u = 0; u < KV; u++)
+                if (active[u]) {  // a converged column keeps its last product
+                    const double y = MODE == BS_RESID ? w[u] - sum[u] : sum[u];
+                    Y[q + u] = y;
+                    acc[u] += MODE == BS_RESID ? y * y : w[u] * y;
+                }
         }
     }
-    if (block_reduce_cols<1>(acc, k, slot, tot)) {
+    if (block_reduce_cols<KV>(acc, kt, slot, tot)) {
         if (threadIdx.x < k) {
-            KState *s = st + threadIdx.x;
-            const double d = tot[threadIdx.x];
+            const int col = threadIdx.x;
+            KState *s = st + col;
+            const double d = tot[col % KV * kt + col / KV];
             if (MODE == BS_RESID) {
                 s->sc[S_RES0SQ] = d;
             } else if (s->done == 0) {
@@ -152,12 +205,22 @@ __global__ void __launch_bounds__(BATCH_THREADS) k_bspmv(int n, int k, const int
         if (threadIdx.x == 0) batch_set_all_done(st, k, all_done);
     }
 }
+template <int MODE>
+inline void launch_bspmv(int G, int TB, cudaStream_t s, int n, int k, const DevCsr &A, const double *X, double *Y,
+                         const double *W, KState *st, int *all_done, RedSlot sl)
+{
+    if (k % 2 == 0) k_bspmv<MODE, 2><<<G, TB, 0, s>>>(n, k, A.rp, A.ci, A.v, X, Y, W, st, all_done, sl);
+    else k_bspmv<MODE, 1><<<G, TB, 0, s>>>(n, k, A.rp, A.ci, A.v, X, Y, W, st, all_done, sl);
+}
 
 // ---------------------------------------------------------------- batched PCG vector ops
 // The element operations are those of OpCgmInit / OpCgmUpdate / OpDotRZ /
 // OpPUpdate (same expressions, so the same bits for the same scalars).
+// Bound by bytes in flight: with one element at a time the x and r update of
+// eight columns at 96^3 took 88 us and r.z 42 us, with BPCG_U 58 and 31.
+constexpr int BPCG_U = 4;  // elements of each vector in flight per thread
 template <int OP>
-__global__ void __launch_bounds__(BATCH_THREADS) k_bpcg(int n, int k, KState *st, int *all_done, double *X,
+__global__ void __launch_bounds__(BATCH_THREADS, BATCH_CTAS) k_bpcg(int n, int k, KState *st, int *all_done, double *X,
                                                        double *R, double *Z, double *P, const double *AP, RedSlot slot)
 {
     constexpr int NV = OP == 0 ? 2 : (OP == 3 ? 0 : 1);
@@ -171,23 +234,42 @@ __global__ void __launch_bounds__(BATCH_THREADS) k_bpcg(int n, int k, KState *st
     if (OP == 1) a = st[c].sc[S_ALPHA];
     if (OP == 3) a = st[c].sc[S_BETA];
     if (active) {
-        for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < m; q += (long)gridDim.x * blockDim.x) {
-            if (OP == 0) {  // init: acc0 = r.r, acc1 = r.z ; p = z
-                const double ri = R[q], zi = Z[q];
-                acc[0] += ri * ri;
-                acc[1] += ri * zi;
-                P[q] = zi;
-            } else if (OP == 1) {  // x += alpha p ; r -= alpha Ap ; acc r.r
-                const double minalpha = -a;
-                X[q] = X[q] + a * P[q];
-                const double ri = R[q] + minalpha * AP[q];
-                R[q] = ri;
-                acc[0] += ri * ri;
-            } else if (OP == 2) {  // acc r.z
-                acc[0] += R[q] * Z[q];
-            } else {  // p = beta p + z
-                const double t = a * P[q];
-                P[q] = t + Z[q];
+        // BPCG_U elements at a time, all loads before the first store
+        const long stride = (long)gridDim.x * blockDim.x;
+        for (long q0 = blockIdx.x * (long)blockDim.x + threadIdx.x; q0 < m; q0 += BPCG_U * stride) {
+            double x[BPCG_U], r[BPCG_U], z[BPCG_U], p[BPCG_U], ap[BPCG_U];
+#pragma unroll
+            for (int u = 0; u < BPCG_U; u++) {
+                const long q = q0 + u * stride;
+                x[u] = r[u] = z[u] = p[u] = ap[u] = 0.0;
+                if (q < m) {
+                    if (OP == 1) x[u] = X[q];
+                    if (OP != 3) r[u] = R[q];
+                    if (OP != 1) z[u] = Z[q];
+                    if (OP == 1 || OP == 3) p[u] = P[q];
+                    if (OP == 1) ap[u] = AP[q];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < BPCG_U; u++) {
+                const long q = q0 + u * stride;
+                if (q >= m) break;
+                if (OP == 0) {  // init: acc0 = r.r, acc1 = r.z ; p = z
+                    acc[0] += r[u] * r[u];
+                    acc[1] += r[u] * z[u];
+                    P[q] = z[u];
+                } else if (OP == 1) {  // x += alpha p ; r -= alpha Ap ; acc r.r
+                    const double minalpha = -a;
+                    X[q] = x[u] + a * p[u];
+                    const double ri = r[u] + minalpha * ap[u];
+                    R[q] = ri;
+                    acc[0] += ri * ri;
+                } else if (OP == 2) {  // acc r.z
+                    acc[0] += r[u] * z[u];
+                } else {  // p = beta p + z
+                    const double t = a * p[u];
+                    P[q] = t + z[u];
+                }
             }
         }
     }
@@ -562,14 +644,14 @@ struct BatchPcg {
         int *ad = S.all_done.p;
         const RedSlot sl = S.slot();
         if (M.type != PC_NONE && M.type != PC_JACOBI) BP.ensure(M, n, k, s);  // before any capture
-        const int G = batch_grid(), TB = batch_block(k);
-        k_bspmv<BS_RESID><<<G, TB, 0, s>>>(n, k, A.rp, A.ci, A.v, X, R, B, st, ad, sl);
+        const int G = batch_grid_for(n, k), TB = batch_block(k);
+        launch_bspmv<BS_RESID>(G, TB, s, n, k, A, X, R, B, st, ad, sl);
         batch_apply(M, BP, k, R, Z, ad, s);
         k_bpcg<0><<<G, TB, 0, s>>>(n, k, st, ad, X, R, Z, P, AP, sl);
         check_launch();
         if (launches) *launches += 5;
         auto body = [&]() {
-            k_bspmv<BS_DOT_SIGMA><<<G, TB, 0, s>>>(n, k, A.rp, A.ci, A.v, P, AP, P, st, ad, sl);
+            launch_bspmv<BS_DOT_SIGMA>(G, TB, s, n, k, A, P, AP, P, st, ad, sl);
             k_bpcg<1><<<G, TB, 0, s>>>(n, k, st, ad, X, R, Z, P, AP, sl);
             batch_apply(M, BP, k, R, Z, ad, s);
             k_bpcg<2><<<G, TB, 0, s>>>(n, k, st, ad, X, R, Z, P, AP, sl);

@@ -302,19 +302,36 @@ int xs_plan_debug_break_dependency(xs_plan_t p, int position, int enable)
         int row = 0;
         XS_CUDA(cudaMemcpy(&row, L.perm.p + position, sizeof(int), cudaMemcpyDeviceToHost));
         // the saved entry may be an encoded (negative) chunk-local slot
-        static thread_local int saved = 0, saved_pos = 0;
+        static thread_local int saved = 0;
+        static thread_local uint32_t saved_dep[2] = {0, 0};
         static thread_local bool have_saved = false;
         if (enable) {
             if (!have_saved) {
                 XS_CUDA(cudaMemcpy(&saved, L.pci.p + k[0], sizeof(int), cudaMemcpyDeviceToHost));
-                if (L.ppos.p) XS_CUDA(cudaMemcpy(&saved_pos, L.ppos.p + k[0], sizeof(int), cudaMemcpyDeviceToHost));
+                if (L.clu_c) {
+                    XS_CUDA(cudaMemcpy(&saved_dep[0], L.clu_dep.p + k[0], sizeof(uint32_t), cudaMemcpyDeviceToHost));
+                    XS_CUDA(cudaMemcpy(&saved_dep[1], L.clu_last.p + position, sizeof(uint32_t), cudaMemcpyDeviceToHost));
+                }
             }
             have_saved = true;
             XS_CUDA(cudaMemcpy(L.pci.p + k[0], &row, sizeof(int), cudaMemcpyHostToDevice));  // waits on itself
-            if (L.ppos.p) XS_CUDA(cudaMemcpy(L.ppos.p + k[0], &position, sizeof(int), cudaMemcpyHostToDevice));
+            if (L.clu_c) {
+                std::vector<int> ls(L.nlevels + 1);
+                XS_CUDA(cudaMemcpy(ls.data(), L.lstart.p, sizeof(int) * ls.size(), cudaMemcpyDeviceToHost));
+                const int l = (int)(std::upper_bound(ls.begin(), ls.end(), position) - ls.begin()) - 1;
+                const int j = position - ls[l], w = ls[l + 1] - ls[l], c = (int)((long)j * L.clu_c / w);
+                int slot = 0;
+                XS_CUDA(cudaMemcpy(&slot, L.clu_lslot.p + (size_t)l * L.clu_c + c, sizeof(int), cudaMemcpyDeviceToHost));
+                const uint32_t own = clu_pack((uint32_t)c, (uint32_t)(slot + j - clu_part(w, c, L.clu_c)));
+                XS_CUDA(cudaMemcpy(L.clu_dep.p + k[0], &own, sizeof(own), cudaMemcpyHostToDevice));
+                XS_CUDA(cudaMemcpy(L.clu_last.p + position, &own, sizeof(own), cudaMemcpyHostToDevice));
+            }
         } else if (have_saved) {
             XS_CUDA(cudaMemcpy(L.pci.p + k[0], &saved, sizeof(int), cudaMemcpyHostToDevice));
-            if (L.ppos.p) XS_CUDA(cudaMemcpy(L.ppos.p + k[0], &saved_pos, sizeof(int), cudaMemcpyHostToDevice));
+            if (L.clu_c) {
+                XS_CUDA(cudaMemcpy(L.clu_dep.p + k[0], &saved_dep[0], sizeof(uint32_t), cudaMemcpyHostToDevice));
+                XS_CUDA(cudaMemcpy(L.clu_last.p + position, &saved_dep[1], sizeof(uint32_t), cudaMemcpyHostToDevice));
+            }
             have_saved = false;
         }
     });

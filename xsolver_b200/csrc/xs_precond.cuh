@@ -59,7 +59,7 @@ struct PrecondDev {
         }
         if (L.lined) line_xchg_ensure(lx64, L.lines.g, 1, s);
         if (U.lined) line_xchg_ensure(ux64, U.lines.g, 1, s);
-        if (L.ppos.p && y64.n != (size_t)n) y64.alloc(n);
+        if (L.clu_c && y64.n != (size_t)n) y64.alloc(n);
     }
     void ensure_buffers32(cudaStream_t s)
     {
@@ -72,7 +72,7 @@ struct PrecondDev {
         }
         if (L.lined) line_xchg_ensure(lx32, L.lines.g, 1, s);
         if (U.lined) line_xchg_ensure(ux32, U.lines.g, 1, s);
-        if (L.ppos.p && y32.n != (size_t)n) y32.alloc(n);
+        if (L.clu_c && y32.n != (size_t)n) y32.alloc(n);
     }
     // temporaries of the Jacobi-sweep mode
     void ensure_sweep_buffers(bool need32)

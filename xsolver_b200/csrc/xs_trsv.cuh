@@ -920,7 +920,11 @@ struct TriDev {
     int lub_rows = 0, lub_entries = 0;  // batch limits the list was built with
     int max_level_rows = 0;  // widest dependency level (level layout)
     DBuf<int> lub;
-    DBuf<int> ppos;  // level layout: dependency position of each entry (k_lu_cluster)
+    // level layout, cluster solve (k_lu_cluster): see CluArgs; clu_c = 0: none
+    int clu_c = 0, clu_slots = 0;
+    DBuf<int> clu_lslot;
+    DBuf<uint32_t> clu_dep, clu_last;
+    CluArgs clu_args() const { return CluArgs{nlevels, lstart.p, clu_lslot.p, clu_dep.p, clu_last.p}; }
     bool tiled = false;
     int ntiles = 0, tile_elems = 0;  // tile_elems: shared-memory values per box (rows + halo)
     int t_max_rows = 0, t_max_halo = 0, t_max_entries = 0;
@@ -1267,17 +1271,36 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
         k_pos_entries<<<g, 256, 0, s>>>(n, upper, T.perm.p, T.prp.p, T.rp_nat.p, T.ci_nat.p, T.src_nat.p, T.pci.p,
                                         T.src.p);
         check_launch();
-        T.ppos.free();
-        if (T.nnz && n <= CLU_MAX * (int)(CLU_SMEM_MAX / sizeof(float))) {  // sizes the cluster solve can serve
-            DBuf<int> pos_of;
-            pos_of.alloc(n);
-            T.ppos.alloc(m);
-            k_inverse_perm<<<g, 256, 0, s>>>(n, T.perm.p, pos_of.p);
-            k_entry_positions<<<g, 256, 0, s>>>(T.nnz, T.pci.p, pos_of.p, T.ppos.p);
-            check_launch();
-            XS_CUDA(cudaStreamSynchronize(s));  // before the temporary is freed
-        }
         T.lstart.alloc(P.nlevels + 1, 4); T.lstart.upload(P.lstart.data(), P.nlevels + 1, s);
+        // tables of the cluster solve, for sizes it can serve
+        T.clu_c = 0;
+        T.clu_lslot.free(); T.clu_dep.free(); T.clu_last.free();
+        const int C = n <= CLU_MAX * (int)(CLU_SMEM_MAX / sizeof(float)) ? clu_size<double, double, double>() : 0;
+        if (C > 0 && T.nnz && P.nlevels > 0) {
+            std::vector<int> lslot((size_t)P.nlevels * C), used(C, 0);
+            for (int l = 0; l < P.nlevels; l++) {
+                const int w = P.lstart[l + 1] - P.lstart[l];
+                for (int c = 0; c < C; c++) {
+                    lslot[(size_t)l * C + c] = used[c];
+                    used[c] += clu_part(w, c + 1, C) - clu_part(w, c, C);
+                }
+            }
+            T.clu_slots = *std::max_element(used.begin(), used.end());
+            if (T.clu_slots < 65536) {
+                T.clu_c = C;
+                T.clu_lslot.alloc(lslot.size()); T.clu_lslot.upload(lslot.data(), lslot.size(), s);
+                T.clu_dep.alloc(m);
+                T.clu_last.alloc(n);
+                DBuf<uint32_t> where;
+                DBuf<int> level;
+                where.alloc(n);
+                level.alloc(n);
+                k_clu_rows<<<g, 256, 0, s>>>(n, P.nlevels, C, T.perm.p, T.lstart.p, T.clu_lslot.p, where.p, level.p);
+                k_clu_entries<<<g, 256, 0, s>>>(n, T.prp.p, T.pci.p, where.p, level.p, T.clu_dep.p, T.clu_last.p);
+                check_launch();
+                XS_CUDA(cudaStreamSynchronize(s));  // before the temporaries are freed
+            }
+        }
         T.max_level_rows = 0;
         for (int l = 0; l < P.nlevels; l++) T.max_level_rows = std::max(T.max_level_rows, P.lstart[l + 1] - P.lstart[l]);
         // level batches of the staged single-CTA solve (systems it serves only)
@@ -1732,10 +1755,8 @@ inline void launch_lu_block(const TriDev &L, const TriDev &U, const DT *dinv, co
 template <typename VT, typename FT, typename DT>
 inline int lu_cluster_slots(const TriDev &L, const TriDev &U)
 {
-    if (!trsv_tuning().cluster || !L.ppos.p || !U.ppos.p) return 0;
-    const int C = clu_size<VT, FT, DT>();
-    if (C == 0) return 0;
-    const int groups = (L.n + 31) / 32, slots = (groups + C - 1) / C * 32;
+    if (!trsv_tuning().cluster || L.clu_c == 0 || L.clu_c != U.clu_c || clu_size<VT, FT, DT>() < L.clu_c) return 0;
+    const int slots = std::max(L.clu_slots, U.clu_slots);
     return (size_t)slots * sizeof(VT) <= CLU_SMEM_MAX ? slots : 0;
 }
 
@@ -1743,12 +1764,11 @@ template <typename VT, typename FT, typename DT>
 inline void launch_lu_cluster(const TriDev &L, const TriDev &U, int slots, const DT *dinv, const VT *x, VT *y, VT *z,
                               const int *done_flag, int *err, cudaStream_t s)
 {
-    const int C = clu_size<VT, FT, DT>();
-    int cshift = 0;
-    while ((1 << cshift) < C) cshift++;
-    // about CLU_AHEAD levels' rows in flight
+    const int C = L.clu_c;
+    // warps for the chunks of about CLU_AHEAD levels
     const long width = std::max(1L, (long)L.n / std::max(1, std::max(L.nlevels, U.nlevels)));
-    const int nw = (int)std::max(1L, std::min<long>(CLU_WARPS_MAX, (CLU_AHEAD * width + 32 * C - 1) / (32 * C)));
+    const long chunks = (width / C + 31) / 32;
+    const int nw = (int)std::max(2L, std::min<long>(CLU_WARPS_MAX, CLU_AHEAD * chunks));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(C);
     cfg.blockDim = dim3(32 * nw);
@@ -1762,9 +1782,8 @@ inline void launch_lu_cluster(const TriDev &L, const TriDev &U, int slots, const
     at[1].val.programmaticStreamSerializationAllowed = pdl_tuning().enabled ? 1 : 0;
     cfg.attrs = at;
     cfg.numAttrs = 2;
-    if (cudaLaunchKernelEx(&cfg, k_lu_cluster<VT, FT, DT>, L.args<FT>(), (const int *)L.ppos.p, U.args<FT>(),
-                           (const int *)U.ppos.p, dinv, x, y, z, done_flag, err, (uint32_t)C, (uint32_t)cshift,
-                           slots) != cudaSuccess)
+    if (cudaLaunchKernelEx(&cfg, k_lu_cluster<VT, FT, DT>, L.args<FT>(), L.clu_args(), U.args<FT>(), U.clu_args(), dinv,
+                           x, y, z, done_flag, err, C, slots) != cudaSuccess)
         throw Status(XS_ERR_CUDA);
 }
 

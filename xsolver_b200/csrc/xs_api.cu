@@ -27,6 +27,7 @@
 #include "xs_batch.cuh"
 #include "xs_mtx.cuh"
 #include "xs_hostilu.h"
+#include "xs_hostio.cuh"
 
 namespace xs {
 
@@ -482,6 +483,7 @@ struct Handle {
     bool have_solution = false;
     // several right-hand sides at once (xs_solve_batch, xs_adjoint_batch)
     BatchRuntime batch;
+    HostIo io;  // large copies from and to the caller's arrays
 
     Handle()
     {
@@ -601,7 +603,7 @@ static void update_values(Handle &h, const double *v)
     if (h.vperm.empty()) {
         // straight from the caller's buffer (a DMA when it is pinned); the
         // host copy is refreshed only if host-side code needs it later
-        h.A.v.upload(v, h.nnz, h.s);
+        h.io.upload(h.A.v.p, v, sizeof(double) * h.nnz, h.s);
         h.hv_stale = true;
     } else {
         for (long k = 0; k < h.nnz; k++) h.hv[k] = v[h.vperm[k]];
@@ -1479,16 +1481,15 @@ static void solve_host(Handle &h, const double *rhs, double *sol)
     if (!rhs || !sol) throw Status(XS_ERR_INVALID);
     const int n = h.n;
     double *b = h.vpool64.get(3, n), *x = h.vpool64.get(4, n);
-    XS_CUDA(cudaMemcpyAsync(b, rhs, sizeof(double) * n, cudaMemcpyHostToDevice, h.s));
-    XS_CUDA(cudaMemcpyAsync(x, sol, sizeof(double) * n, cudaMemcpyHostToDevice, h.s));
+    h.io.upload(b, rhs, sizeof(double) * n, h.s);
+    h.io.upload(x, sol, sizeof(double) * n, h.s);
     int status = XS_OK;
     try {
         solve_device(h, b, x);
     } catch (Status &st) {
         status = st.code;
     }
-    XS_CUDA(cudaMemcpyAsync(sol, x, sizeof(double) * n, cudaMemcpyDeviceToHost, h.s));
-    XS_CUDA(cudaStreamSynchronize(h.s));
+    h.io.download(sol, x, sizeof(double) * n, h.s);
     if (status) throw Status(status);
 }
 
@@ -1597,7 +1598,7 @@ static void adjoint_solve(Handle &h, const double *dLdx, double *dLdb, double *d
     const int n = h.n;
     clear_dev_err(h);
     if (a.lam.n != (size_t)n) { a.lam.alloc(n); a.rhs.alloc(n); }
-    a.rhs.upload(dLdx, n, h.s);
+    h.io.upload(a.rhs.p, dLdx, sizeof(double) * n, h.s);
     XS_CUDA(cudaMemsetAsync(a.lam.p, 0, sizeof(double) * n, h.s));
     // backward solve with the forward method (FP64), transposed operator/preconditioner
     prepare_state(h, h.maxiter, h.tol, h.abstol, true);
@@ -1616,9 +1617,9 @@ static void adjoint_solve(Handle &h, const double *dLdx, double *dLdb, double *d
     }
     k_adjoint_grad<<<geom().sms * 4, 256, 0, h.s>>>(n, h.A.rp.p, h.A.ci.p, a.lam.p, a.x_last.p, db, dA);
     check_launch();
-    if (dLdb) gb.download(dLdb, n, h.s);
+    if (dLdb) h.io.download(dLdb, gb.p, sizeof(double) * n, h.s);
     if (dLdA) {
-        if (h.vperm.empty()) gA.download(dLdA, h.nnz, h.s);
+        if (h.vperm.empty()) h.io.download(dLdA, gA.p, sizeof(double) * h.nnz, h.s);
         else {
             std::vector<double> t(h.nnz);
             gA.download(t.data(), h.nnz, h.s);
@@ -1678,9 +1679,9 @@ static void solve_batch(Handle &h, int k, const double *rhs, double *sol)
     BatchRuntime &R = h.batch;
     if (R.bB.n != (size_t)m) { R.bB.alloc(m); R.bX.alloc(m); R.tmp.alloc(m); }
     const int g = geom().sms * 4;
-    R.tmp.upload(rhs, m, h.s);
+    h.io.upload(R.tmp.p, rhs, sizeof(double) * m, h.s);
     k_interleave<<<g, 256, 0, h.s>>>(n, k, R.tmp.p, R.bB.p);
-    R.tmp.upload(sol, m, h.s);  // x0 of every column
+    h.io.upload(R.tmp.p, sol, sizeof(double) * m, h.s);  // x0 of every column
     k_interleave<<<g, 256, 0, h.s>>>(n, k, R.tmp.p, R.bX.p);
     check_launch();
     R.S.prepare(k, h.maxiter, h.tol, h.abstol, h.s);
@@ -1694,8 +1695,7 @@ static void solve_batch(Handle &h, int k, const double *rhs, double *sol)
     XS_CUDA(cudaEventRecord(e1, h.s));
     k_deinterleave<<<g, 256, 0, h.s>>>(n, k, R.bX.p, R.tmp.p);
     check_launch();
-    R.tmp.download(sol, m, h.s);
-    XS_CUDA(cudaStreamSynchronize(h.s));
+    h.io.download(sol, R.tmp.p, sizeof(double) * m, h.s);
     float ms = 0;
     cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
@@ -1749,9 +1749,9 @@ static void adjoint_batch(Handle &h, int k, const double *X, const double *G, do
     if (R.bB.n != (size_t)m) { R.bB.alloc(m); R.bX.alloc(m); R.tmp.alloc(m); }
     if (R.bY.n != (size_t)m) R.bY.alloc(m);
     const int g = geom().sms * 4;
-    R.tmp.upload(G, m, h.s);
+    h.io.upload(R.tmp.p, G, sizeof(double) * m, h.s);
     k_interleave<<<g, 256, 0, h.s>>>(n, k, R.tmp.p, R.bB.p);  // right-hand sides dL/dx
-    R.tmp.upload(X, m, h.s);
+    h.io.upload(R.tmp.p, X, sizeof(double) * m, h.s);
     k_interleave<<<g, 256, 0, h.s>>>(n, k, R.tmp.p, R.bY.p);  // forward solutions
     check_launch();
     XS_CUDA(cudaMemsetAsync(R.bX.p, 0, sizeof(double) * m, h.s));  // lambda0 = 0
@@ -1776,9 +1776,9 @@ static void adjoint_batch(Handle &h, int k, const double *X, const double *G, do
     k_adjoint_grad_multi<<<g, 256, 0, h.s>>>(n, k, h.nnz, h.A.rp.p, h.A.ci.p, R.bX.p, R.bY.p, db, dA);
     check_launch();
     XS_CUDA(cudaEventRecord(e1, h.s));
-    if (DB) R.gb.download(DB, m, h.s);
+    if (DB) h.io.download(DB, R.gb.p, sizeof(double) * m, h.s);
     if (DA) {
-        if (h.vperm.empty()) R.gA.download(DA, (size_t)k * h.nnz, h.s);
+        if (h.vperm.empty()) h.io.download(DA, R.gA.p, sizeof(double) * (size_t)k * h.nnz, h.s);
         else {
             std::vector<double> t((size_t)k * h.nnz);
             R.gA.download(t.data(), t.size(), h.s);

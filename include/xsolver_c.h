@@ -454,7 +454,8 @@ int xs_set_vector_fusion(int enable);
 int xs_set_persistent_iteration(int enable);
 /* Box-scheduled exact triangular solves (see xs_tri_tiles): enable = 1
  * (default) uses them for triangles of at least min_rows rows (default
- * 65536, at least 8) whose pattern fits a grid, with boxes of tx*ty*tz
+ * 65536, at least 8) whose pattern fits a grid and is not line-scheduled
+ * (xs_set_trsv_lines), with boxes of tx*ty*tz
  * sheared grid steps (default 16*16*8, halved along the longest side until
  * a box's staged data fits in shared memory; triangles averaging at least 20
  * entries per row, such as ParILUT fill of 27-point operators, start from
@@ -467,11 +468,11 @@ int xs_set_persistent_iteration(int enable);
 int xs_set_trsv_tiles(int enable, int tx, int ty, int tz, int min_rows);
 /* Line-scheduled exact triangular solves: mode 1 (default) uses them instead
  * of boxes, level order or the single-CTA solve for triangles of at least
- * min_rows rows (default 512) whose entries lie on at most 32 diagonals of a
- * grid with little padding (stencil ILU(0), ParILUT fill of a stencil),
- * unless xs_set_trsv_tiles turned grid schedules off or set a box size;
- * 2 also with a box size set; 0 never.  Results are bitwise the same.
- * Fixed when a preconditioner is built. */
+ * min_rows rows (default 512, and 4096 for 7-point ones) whose entries lie on
+ * at most 32 diagonals of a grid with little padding (stencil ILU(0), ParILUT
+ * fill of a stencil), unless xs_set_trsv_tiles turned grid schedules off or
+ * set a box size; 2 also with a box size set; 0 never.  Results are bitwise
+ * the same.  Fixed when a preconditioner is built. */
 int xs_set_trsv_lines(int mode, int min_rows);
 /* Exact LU solves of patterns without a grid schedule on one thread-block
  * cluster, the solution vector in its distributed shared memory (FP64 up to
@@ -483,7 +484,8 @@ int xs_set_trsv_cluster(int enable);
  * that walks the dependency levels with a block barrier between them
  * (bitwise the same result as the sync-free solve, without its cross-SM
  * hand-off per level).  0 disables it; default: no row limit beyond the
- * shared-memory one.  Environment XS_TRSV_BLOCK_ROWS sets it at first use. */
+ * shared-memory one, but systems of at least 4096 rows go to the cluster
+ * solve where it serves them (xs_set_trsv_cluster).  Environment XS_TRSV_BLOCK_ROWS sets it at first use. */
 int xs_set_trsv_block_rows(int max_rows);
 /* Single-CTA LU solve form: 1 (default) copies whole dependency levels, in
  * batches of up to 512 rows and 2048 entries, into shared memory with

@@ -2041,7 +2041,7 @@ int xs_set_trsv_lines(int mode, int min_rows)
     return guarded([&] {
         if (mode < 0 || mode > 2 || (mode && min_rows < 8)) throw Status(XS_ERR_INVALID);
         tile_tuning().lines = mode;
-        if (mode) tile_tuning().line_min_rows = min_rows;
+        if (mode) tile_tuning().line_min_rows = tile_tuning().line_min_rows_7pt = min_rows;
     });
 }
 

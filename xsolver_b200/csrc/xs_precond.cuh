@@ -153,14 +153,15 @@ struct PrecondDev {
     void apply_exact(const VT *x, VT *z, const int *done_flag, cudaStream_t s)
     {
         if (!L.vals<FT>() || !U.vals<FT>()) throw Status(XS_ERR_ORDER);  // copies not built for this configuration
-        if (lu_block_ok<VT>(L, U)) {
+        const int slots = lu_cluster_slots<VT, FT, VT>(L, U);
+        if (lu_block_ok<VT>(L, U, slots > 0)) {
             const VT *dinv;
             if constexpr (std::is_same<VT, double>::value) dinv = U.dinv64.p;
             else dinv = U.dinv32.p;
             launch_lu_block<VT, FT, VT>(L, U, dinv, x, z, done_flag, s);
             return;
         }
-        if (const int slots = lu_cluster_slots<VT, FT, VT>(L, U)) {
+        if (slots) {
             const VT *dinv;
             if constexpr (std::is_same<VT, double>::value) dinv = U.dinv64.p;
             else dinv = U.dinv32.p;

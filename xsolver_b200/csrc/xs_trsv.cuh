@@ -1154,7 +1154,8 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
         Trace tr_det("      grid detection", s);
         const bool on_grid = tile_detect(n, rp.data(), ci.data(), upper, G);
         tr_det.stop();
-        if (on_grid && want_lines && line_layout(n, T.nnz, G, geom().sms, H) && !repeats()) {
+        if (on_grid && want_lines && line_layout(n, T.nnz, G, geom().sms, H) &&
+            (H.g.D != 3 || n >= tile_tuning().line_min_rows_7pt) && !repeats()) {
             T.lined = true;
             LinePlan &P = T.lines;
             P.g = H.g;
@@ -1703,10 +1704,14 @@ __global__ void __launch_bounds__(LU_BLOCK_THREADS) k_lu_staged(TrsvArgs<FT> L, 
 }
 
 // whether the single-CTA solve serves this pair of plans for vectors of VT
+// (cluster: the cluster solve serves them too.  It hands over between SMs,
+// but loads and sums on 16 of them: LU solve of a mesh, one CTA / cluster, us:
+// 512 rows 51 / 68, 2,184 127 / 125, 8,000 232 / 217, 18,750 381 / 335)
 template <typename VT>
-inline bool lu_block_ok(const TriDev &L, const TriDev &U)
+inline bool lu_block_ok(const TriDev &L, const TriDev &U, bool cluster)
 {
     const TrsvTuning &t = trsv_tuning();
+    if (cluster && t.block_max_rows == 1 << 30 && L.n >= CLU_MIN_ROWS) return false;
     return !L.chunked && !U.chunked && L.n > 0 && L.n <= t.block_max_rows &&
            (size_t)L.n * sizeof(VT) <= LU_BLOCK_SMEM_MAX && L.lstart.p && U.lstart.p;
 }

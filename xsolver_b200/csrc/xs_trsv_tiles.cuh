@@ -82,7 +82,13 @@ struct TileTuning {
     int blocks_per_sm = 4;
     int user_box = 0;  // tx/ty/tz set by the caller (xs_set_trsv_tiles, XS_TRSV_TILES): no dense-row default
     int lines = 1;  // line schedule where the pattern qualifies: 1 unless the caller set a box size, 2 also then
+    // smallest systems on lines.  Below, one CTA walks the levels as fast; a
+    // 7-point triangle has short lines and few levels, so it starts later
+    // (LU solve in one CTA / on lines, us: 24^2 33 / 25, 40^2 54 / 36,
+    // 27-point 8^3 76 / 76, 10^3 105 / 79, 16^3 179 / 100; 7-point 10^3 25 / 30,
+    // 12^3 29 / 30, 16^3 41 / 34, 32*32*4 54 / 38, 28^3 164 / 66)
     int line_min_rows = 512;
+    int line_min_rows_7pt = 4096;
 };
 // Triangles with at least this many entries per row on average start from
 // TILE_DENSE_BOX boxes instead of tx/ty/tz: small boxes, long along x, four

@@ -144,3 +144,37 @@ def test_whole_solve_matches_sync_free(cuda):
             res.append((S.solve(b), S.resvec()))
             S.close()
     assert np.array_equal(res[0][0], res[1][0]) and np.array_equal(res[0][1], res[1][1])
+
+
+@pytest.mark.parametrize("n", [4095, 4096, 4097, 25600, 25601])
+def test_default_choice_bitwise_vs_oracle(cuda, n):
+    """Around the sizes where the solve in one CTA hands over to the cluster,
+    and where its shared memory ends: the default's result is the oracle's."""
+    from xsolver_b200.api import Plan
+
+    A = mesh(n, 60, 3, n)
+    x = st.rhs_uniform(n, 3)
+    for z in _lusolve(Plan(A).factor("ilu0"), x, cuda, reps=2):
+        assert np.array_equal(z, oracle.lusolve(oracle.ilu0(A), x))
+
+
+@pytest.mark.parametrize("shape", [(15, 16, 17), (16, 16, 16), (8, 8, 8)])
+def test_default_choice_of_small_grids(cuda, shape):
+    """7-point grids around the smallest one on lines."""
+    from xsolver_b200.api import Plan
+
+    nx, ny, nz = shape
+    i = np.arange(nx * ny * nz)
+    x, y, z = i % nx, i // nx % ny, i // (nx * ny)
+    r, c = [i], [i]
+    for d, on in ((1, x + 1 < nx), (nx, y + 1 < ny), (nx * ny, z + 1 < nz)):
+        r += [i[on], i[on] + d]
+        c += [i[on] + d, i[on]]
+    r, c = np.concatenate(r), np.concatenate(c)
+    o = np.lexsort((c, r))
+    r, c = r[o], c[o]
+    v = np.where(r == c, 6.5, -np.random.default_rng(1).uniform(0.3, 1.0, r.size))
+    A = CSRMatrix(i.size, np.concatenate([[0], np.cumsum(np.bincount(r))]), c, v)
+    b = st.rhs_uniform(A.n, 3)
+    for w in _lusolve(Plan(A).factor("ilu0"), b, cuda, reps=2):
+        assert np.array_equal(w, oracle.lusolve(oracle.ilu0(A), b))

@@ -1,0 +1,105 @@
+"""One handle or plan given another matrix or another kind of factor.
+
+The reference keeps one global matrix and preconditioner and builds them
+anew on every xsolver_mat_setup and preconditioner setup
+(hip/xsolver_c.cpp:274-292), so a program may change both at any time.  Here
+a handle rebuilds its plans in place, and the schedule of the exact
+triangular solves follows the pattern: whatever the handle did before, every
+result has to equal that of a handle that did nothing else, bit for bit."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from test_gpu_cluster import mesh
+from test_lines import P7, _stencil
+from xsolver_b200 import stencils as st
+
+pytestmark = pytest.mark.gpu
+
+
+def _setup(S, A):
+    """A new matrix on the handle of S."""
+    from xsolver_b200.api import check
+
+    S.A, S._rp, S._ci, S._v = A, A.rowptr, A.colidx, A.val
+    p = lambda a, t: a.ctypes.data_as(C.POINTER(t))  # noqa: E731
+    check(S._L.xs_mat_setup(S.h, A.n, p(S._rp, C.c_int), p(S._ci, C.c_int), p(S._v, C.c_double), 0), "xs_mat_setup")
+
+
+def _fresh(A, ksp="bicgstab", pc="ilu0"):
+    from xsolver_b200.api import Solver
+
+    return Solver(A).ksp_settype(ksp).ksp_setoption(1e-10, 300, 20).pc_settype(pc)
+
+
+class tuning:
+    """Lines off (boxes from 65536 rows) and / or the single-CTA and cluster solves off."""
+
+    def __init__(self, lines=1, one_cta=1):
+        self.lines, self.one_cta = lines, one_cta
+
+    def __enter__(self):
+        from xsolver_b200 import _lib
+
+        L = _lib.lib()
+        if not self.lines:
+            L.xs_set_trsv_lines(0, 0)
+        if not self.one_cta:
+            L.xs_set_trsv_block_rows(0)
+            L.xs_set_trsv_cluster(0)
+
+    def __exit__(self, *exc):
+        from xsolver_b200 import _lib
+
+        L = _lib.lib()
+        L.xs_set_trsv_lines(1, 512)
+        L.xs_set_trsv_block_rows(1 << 30)
+        L.xs_set_trsv_cluster(1)
+
+
+def _patterns():
+    """(matrix, tuning at its analysis): cluster, lines, boxes, one CTA, sync-free."""
+    M, G, S = mesh(9000, 300, 3, 1), _stencil((24, 25, 26), P7), mesh(300, 20, 2, 2)
+    B = _stencil((41, 41, 41), P7)
+    return {"cluster": (M, {}), "lines": (G, {}), "boxes": (B, dict(lines=0)), "one_cta": (S, {}),
+            "sync_free": (M, dict(one_cta=0))}
+
+
+@pytest.mark.parametrize("order", [("cluster", "lines", "one_cta", "cluster"), ("one_cta", "lines", "cluster"),
+                                   ("cluster", "boxes", "cluster", "lines", "boxes"), ("boxes", "one_cta", "lines")])
+def test_matrices_of_different_schedules_on_one_handle(cuda, order):
+    """A table of an earlier pattern's schedule is never used for a later one."""
+    pats = _patterns()
+    S = None
+    for name in order:
+        A, how = pats[name]
+        b = st.rhs_uniform(A.n, 3)
+        with tuning(**how):
+            if S is None:
+                S = _fresh(A)
+            else:
+                _setup(S, A)
+            x = S.solve(b)
+            N = _fresh(A)
+            assert np.array_equal(x, N.solve(b)), name
+            assert S.usediter == N.usediter
+            N.close()
+    S.close()
+
+
+def test_reference_style_globals_with_a_second_matrix(cuda):
+    """The one global handle of the reference's API: a mesh, then a grid."""
+    from xsolver_b200 import api
+
+    for name in ("cluster", "lines"):
+        A = _patterns()[name][0]
+        b, x = st.rhs_uniform(A.n, 3), np.zeros(A.n)
+        assert api.xsolver_mat_setup(A.n, A.rowptr, A.colidx, A.val) == 0
+        assert api.xsolver_ksp_settype("bicgstab") == 0
+        assert api.xsolver_ksp_setoption(1e-10, 300) == 0
+        assert api.xsolver_pc_settype("ilu0") == 0
+        assert api.xsolver_solve(b, x) == 0
+        r = b - A.to_scipy() @ x
+        assert np.linalg.norm(r) <= 1e-9 * np.linalg.norm(b)
+    assert api.xsolver_free() == 0

@@ -935,6 +935,18 @@ struct TriDev {
     bool lined = false;
     LinePlan lines;
     const int *level_perm() const { return tiled || lined ? lvperm.p : perm.p; }
+    // forget the schedule of an earlier pattern (an analysis is built in
+    // place): no table stays that the new layout does not write, since the
+    // dispatch reads them to see what a triangle has
+    void clear_schedule()
+    {
+        tiled = lined = false;
+        lines = LinePlan();
+        ntiles = nlub = clu_c = clu_slots = max_level_rows = 0;
+        for (DBuf<int> *b : {&t_pos, &t_lvl, &t_lptr, &t_hptr, &t_hrow, &lvperm, &lstart, &lub, &clu_lslot}) b->free();
+        clu_dep.free();
+        clu_last.free();
+    }
     // elements of a value copy in the order of the exact solve
     size_t pos_elems() const { return lined ? (size_t)lines.g.slots() * lines.g.D : (size_t)std::max<long>(nnz, 1); }
     size_t pos_rows() const { return lined ? (size_t)lines.g.slots() : (size_t)n; }
@@ -1129,10 +1141,7 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
     // box layout for patterns on a structured grid (large triangles only);
     // boxes shrink until the rows and halo of one fit in shared memory
     TileHostPlan TP;
-    T.tiled = false;
-    T.lined = false;
-    T.lines = LinePlan();
-    T.t_pos.free(); T.t_lvl.free(); T.t_lptr.free(); T.t_hptr.free(); T.t_hrow.free(); T.lvperm.free();
+    T.clear_schedule();
     const bool want_lines = !T.chunked && tile_tuning().enable && n >= tile_tuning().line_min_rows &&
                             (tile_tuning().lines == 2 || (tile_tuning().lines && !tile_tuning().user_box));
     const bool want_tiles = !T.chunked && tile_tuning().enable && n >= tile_tuning().min_rows;
@@ -1217,7 +1226,7 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
         }
     }
     if (T.lined) {
-        T.perm.free(); T.prp.free(); T.pci.free(); T.src.free(); T.lstart.free();
+        T.perm.free(); T.prp.free(); T.pci.free(); T.src.free();
         if (need_levels) {
             level_analysis();
             T.nlevels = P.nlevels;
@@ -1259,7 +1268,6 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
             T.nlevels = P.nlevels;
             T.lvperm.alloc(n); T.lvperm.upload(P.perm.data(), n, s);
         }
-        T.lstart.free();
         XS_CUDA(cudaStreamSynchronize(s));  // the host plans go out of scope
     } else if (!T.chunked) {
         level_analysis();
@@ -1274,8 +1282,6 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
         check_launch();
         T.lstart.alloc(P.nlevels + 1, 4); T.lstart.upload(P.lstart.data(), P.nlevels + 1, s);
         // tables of the cluster solve, for sizes it can serve
-        T.clu_c = 0;
-        T.clu_lslot.free(); T.clu_dep.free(); T.clu_last.free();
         const int C = n <= CLU_MAX * (int)(CLU_SMEM_MAX / sizeof(float)) ? clu_size<double, double, double>() : 0;
         if (C > 0 && T.nnz && P.nlevels > 0) {
             std::vector<int> lslot((size_t)P.nlevels * C), used(C, 0);
@@ -1302,11 +1308,8 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
                 XS_CUDA(cudaStreamSynchronize(s));  // before the temporaries are freed
             }
         }
-        T.max_level_rows = 0;
         for (int l = 0; l < P.nlevels; l++) T.max_level_rows = std::max(T.max_level_rows, P.lstart[l + 1] - P.lstart[l]);
         // level batches of the staged single-CTA solve (systems it serves only)
-        T.nlub = 0;
-        T.lub.free();
         if ((size_t)n * sizeof(double) <= LU_BLOCK_SMEM_MAX) {
             const TrsvTuning &tu = trsv_tuning();
             int brows = tu.lub_rows, bents = tu.lub_entries;
@@ -1761,6 +1764,7 @@ template <typename VT, typename FT, typename DT>
 inline int lu_cluster_slots(const TriDev &L, const TriDev &U)
 {
     if (!trsv_tuning().cluster || L.clu_c == 0 || L.clu_c != U.clu_c || clu_size<VT, FT, DT>() < L.clu_c) return 0;
+    if (!L.lstart.p || !U.lstart.p) return 0;  // not in level order
     const int slots = std::max(L.clu_slots, U.clu_slots);
     return (size_t)slots * sizeof(VT) <= CLU_SMEM_MAX ? slots : 0;
 }

@@ -103,3 +103,56 @@ def test_reference_style_globals_with_a_second_matrix(cuda):
         r = b - A.to_scipy() @ x
         assert np.linalg.norm(r) <= 1e-9 * np.linalg.norm(b)
     assert api.xsolver_free() == 0
+
+
+def _parts(A, kind="ilu0", **how):
+    """A plan factorised under the given tuning."""
+    from xsolver_b200.api import Plan
+
+    with tuning(**how):
+        return Plan(A).factor(kind, sweeps=3, fill=2.0, droptol=1e-4)
+
+
+def _lusolve(P, x, cuda):
+    import torch
+
+    dx = torch.from_numpy(np.ascontiguousarray(x)).to(cuda)
+    z = torch.full_like(dx, float("nan"))
+    (P.lusolve_batch if dx.dim() == 2 else P.lusolve)(dx, z)
+    P.sync()
+    return z.cpu().numpy()
+
+
+@pytest.mark.parametrize("dtype,cols", [(np.float64, 0), (np.float32, 0), (np.float64, 3)])
+@pytest.mark.parametrize("how", [dict(lines=0, one_cta=0), dict(lines=0)])
+def test_factor_of_another_schedule_on_one_plan(cuda, dtype, cols, how):
+    """ILU(0) on lines and solved, then a threshold factor of another schedule:
+    its first solve does not take what the line solve left in the readiness
+    buffers for finished rows."""
+    A = _stencil((24, 25, 26), P7) if how.get("one_cta") == 0 else _stencil((41, 41, 41), P7)
+    x = st.rhs_uniform(A.n, 5).astype(dtype)
+    if cols:
+        x = np.stack([st.rhs_uniform(A.n, c) for c in range(cols)], 1)
+    P = _parts(A)
+    _lusolve(P, x, cuda)
+    with tuning(**how):
+        P.factor("parilut", sweeps=3, fill=2.0, droptol=1e-4)
+        z = [_lusolve(P, x, cuda) for _ in range(2)]
+        ref = _lusolve(_parts(A, "parilut", **how), x, cuda)
+    assert np.array_equal(z[0], ref) and np.array_equal(z[1], ref)
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_same_pattern_size_with_another_schedule_on_one_handle(cuda, batch):
+    """A grid on lines, then the same system analysed for the sync-free solve."""
+    A = _stencil((24, 25, 26), P7)
+    B = np.stack([st.rhs_uniform(A.n, c) for c in range(3)])
+    solve = (lambda S: S.solve_batch(B)) if batch else (lambda S: S.solve(B[0]))
+    S = _fresh(A, "cg")
+    solve(S)
+    with tuning(lines=0, one_cta=0):
+        _setup(S, A)
+        N = _fresh(A, "cg")
+        assert np.array_equal(solve(S), solve(N))
+    N.close()
+    S.close()

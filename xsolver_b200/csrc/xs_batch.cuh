@@ -464,16 +464,20 @@ struct BatchPrecond {
     DBuf<double> lb, ub;  // readiness buffers, n*k each (NaN sentinel)
     DBuf<unsigned> ticket;
     LineXchg<double> lx, ux;  // line-scheduled triangles
+    ArmedFor armed;           // of lb / ub
     int n = 0, k = 0;
     void ensure(const PrecondDev &M, int nn, int kk, cudaStream_t s)
     {
         if (M.L.lined) line_xchg_ensure(lx, M.L.lines.g, kk, s);
         if (M.U.lined) line_xchg_ensure(ux, M.U.lines.g, kk, s);
-        if (n == nn && k == kk && lb.p) return;
-        n = nn;
-        k = kk;
-        lb.alloc((size_t)n * k);
-        ub.alloc((size_t)n * k);
+        if (n != nn || k != kk || !lb.p) {
+            n = nn;
+            k = kk;
+            lb.alloc((size_t)n * k);
+            ub.alloc((size_t)n * k);
+            armed = ArmedFor();
+        }
+        if (!armed.changed(M.L, M.U)) return;
         k_fill_sentinel<double><<<256, 256, 0, s>>>(lb.p, (int)((size_t)n * k));
         k_fill_sentinel<double><<<256, 256, 0, s>>>(ub.p, (int)((size_t)n * k));
         if (!ticket.p) ticket.alloc(1);

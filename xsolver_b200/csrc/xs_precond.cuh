@@ -31,6 +31,21 @@ __global__ void k_diag_scale(int n, const DT *__restrict__ d, const VT *__restri
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) y[i] = (VT)d[i] * x[i];
 }
 
+// The triangles that a pair of readiness buffers was last filled for.  Two
+// line-scheduled triangles use lbuf as plain storage and leave it unarmed,
+// every other pair polls it; so the buffers are filled again whenever a
+// triangle was rebuilt, before its first solve.
+struct ArmedFor {
+    const void *l = nullptr, *u = nullptr;
+    bool changed(const TriDev &L, const TriDev &U)
+    {
+        if (l == L.layout && u == U.layout && l) return false;
+        l = L.layout;
+        u = U.layout;
+        return true;
+    }
+};
+
 struct PrecondDev {
     int type = PC_NONE;
     int n = 0;
@@ -47,12 +62,16 @@ struct PrecondDev {
     DBuf<float> y32;
     int *err = nullptr;
     bool have_factors = false;
+    ArmedFor armed64, armed32;  // of lbuf / ubuf
 
     void ensure_buffers64(cudaStream_t s)
     {
         if (lbuf64.n != (size_t)n) {
             lbuf64.alloc(n);
             ubuf64.alloc(n);
+            armed64 = ArmedFor();
+        }
+        if (armed64.changed(L, U)) {
             k_fill_sentinel<double><<<256, 256, 0, s>>>(lbuf64, n);
             k_fill_sentinel<double><<<256, 256, 0, s>>>(ubuf64, n);
             check_launch();
@@ -66,6 +85,9 @@ struct PrecondDev {
         if (lbuf32.n != (size_t)n) {
             lbuf32.alloc(n);
             ubuf32.alloc(n);
+            armed32 = ArmedFor();
+        }
+        if (armed32.changed(L, U)) {
             k_fill_sentinel<float><<<256, 256, 0, s>>>(lbuf32, n);
             k_fill_sentinel<float><<<256, 256, 0, s>>>(ubuf32, n);
             check_launch();

@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 
 from test_gpu_cluster import mesh
-from test_lines import P7, _stencil
+from test_lines import P5, P7, _stencil
 from xsolver_b200 import stencils as st
 
 pytestmark = pytest.mark.gpu
@@ -155,4 +155,21 @@ def test_same_pattern_size_with_another_schedule_on_one_handle(cuda, batch):
         N = _fresh(A, "cg")
         assert np.array_equal(solve(S), solve(N))
     N.close()
+    S.close()
+
+
+@pytest.mark.parametrize("first,second", [((96, 96), (16, 25, 25)), ((80, 80), (25, 16, 16))])
+def test_stencils_of_equal_slots_on_one_handle(cuda, first, second):
+    """A 5-point and a 7-point pattern whose line schedules have as many slots
+    (test_equal_slots_of_different_stencils): ILU(0)'s pivot stream of the
+    second is larger by half."""
+    systems = [_stencil(first, P5, 1), _stencil(second, P7, 2)]
+    S = _fresh(systems[0])
+    for A in systems + systems[:1]:
+        if S.A is not A:
+            _setup(S, A)
+        b = st.rhs_uniform(A.n, 3)
+        N = _fresh(A)
+        assert np.array_equal(S.solve(b), N.solve(b))
+        N.close()
     S.close()

@@ -187,3 +187,18 @@ def test_patterns_that_do_not_qualify():
     rp2 = np.zeros(1001, np.int64)
     np.cumsum(np.bincount(rows[keep], minlength=1000), out=rp2[1:])
     assert lines(1000, rp2, ci[keep], False) is None
+
+
+def test_equal_slots_of_different_stencils():
+    """A 5-point and a 7-point schedule of as many slots, whose value streams
+    (slots times diagonals) are of different sizes: what a handle keeps for
+    one pattern cannot be told by the slot count to fit the other."""
+    sizes = []
+    for shape, offs in (((96, 96), P5), ((16, 25, 25), P7), ((80, 80), P5), ((25, 16, 16), P7)):
+        A = _stencil(shape, offs)
+        low = A.colidx < np.repeat(np.arange(A.n), np.diff(A.rowptr))
+        rp = np.concatenate([[0], np.cumsum(low)])[A.rowptr]
+        g = lines(A.n, rp, A.colidx[low], False)
+        sizes.append((g["npatch"] * g["nsteps"] * g["L"], g["D"]))
+    for (sa, da), (sb, db) in (sizes[:2], sizes[2:]):
+        assert sa == sb and (da, db) == (2, 3)

@@ -975,10 +975,9 @@ static void factor_ilu(Handle &h, int kind, int sweeps)
         } else if (on_lines) {
             const LinePlan &P = TL.lines;
             const size_t m = (size_t)P.g.slots();
-            if (h.lilu_mask.n != m) {
-                h.lilu_mask.alloc(m);
-                h.lilu_pv.alloc(m * 2 * P.g.D);
-            }
+            // each by its own size: a 5- and a 7-point pattern can have as many slots
+            if (h.lilu_mask.n != m) h.lilu_mask.alloc(m);
+            if (h.lilu_pv.n != m * 2 * P.g.D) h.lilu_pv.alloc(m * 2 * P.g.D);
             if (h.lilu_a.n != (size_t)n) {
                 h.lilu_a.alloc(n);
                 h.lilu_d.alloc(n);

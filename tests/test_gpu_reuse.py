@@ -173,3 +173,35 @@ def test_stencils_of_equal_slots_on_one_handle(cuda, first, second):
         assert np.array_equal(S.solve(b), N.solve(b))
         N.close()
     S.close()
+
+
+@pytest.mark.parametrize("own", ["parilut", "ilup", "ict"])
+@pytest.mark.parametrize("A", [st.varcoef3d_7pt(24, 1), st.convdiff3d_27pt(14)], ids=lambda A: A.name)
+def test_factors_on_the_matrix_pattern_after_one_on_its_own(cuda, A, own):
+    """ILU(0), a threshold factor, then ILU(0), ParILU and IC(0) on one plan:
+    none of these works on the threshold factor's triangles."""
+    from xsolver_b200.api import Plan
+
+    x = st.rhs_uniform(A.n, 5)
+    P = Plan(A).factor("ilu0")
+    for kind in ("ilu0", "parilu", "ic0"):
+        P.factor(own, sweeps=3, fill=3.0 if own == "parilut" else 20, droptol=1e-4)
+        _lusolve(P, x, cuda)
+        P.factor(kind, sweeps=4)
+        N = Plan(A).factor(kind, sweeps=4)
+        assert np.array_equal(P.lu_values(), N.lu_values(), equal_nan=True), kind
+        assert np.array_equal(_lusolve(P, x, cuda), _lusolve(N, x, cuda), equal_nan=True), kind
+
+
+def test_preconditioners_in_turn_on_one_handle(cuda):
+    A = st.varcoef3d_7pt(24, 1)
+    b, g = st.rhs_uniform(A.n, 3), st.rhs_uniform(A.n, 4)
+    S = _fresh(A, "cg")
+    for pc in ("ilu0", "parilut", "jacobi", "parilut", "ic0", "ilut", "ilu0", "parilu"):
+        S.pc_settype(pc)
+        N = _fresh(A, "cg", pc)
+        assert np.array_equal(S.solve(b), N.solve(b)), pc
+        for a, c in zip(S.adjoint(g), N.adjoint(g)):
+            assert np.array_equal(a, c), pc
+        N.close()
+    S.close()

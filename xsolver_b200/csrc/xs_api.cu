@@ -407,7 +407,7 @@ struct Handle {
     Operator A;
     bool have_matrix = false;
     int format = 0;
-    // pattern analysis of A for factorisations
+    // pattern analysis of A for factorisations (true while M.L and M.U are A's triangles)
     bool analysed = false;
     std::vector<int> huptr;
     DBuf<int> uptr, rowof, ucp, ucpos, flags;
@@ -1143,7 +1143,10 @@ static void build_precond(Handle &h)
             }
             upload_host_factors(h.s, n, F, h.ilut);
         }
-        // factors in the seqilu0 layout on their own pattern
+        // factors in the seqilu0 layout on their own pattern; M.L and M.U are
+        // then no longer A's triangles, which the next factor on A's pattern
+        // has to analyse again
+        h.analysed = false;
         ilut_to_tri(h.s, n, h.ilut, M.L, M.U, need32);
         {
             Trace tr_trim("  scratch pool trim", h.s);

@@ -478,16 +478,16 @@ struct BatchPrecond {
             armed = ArmedFor();
         }
         if (!armed.changed(M.L, M.U)) return;
-        k_fill_sentinel<double><<<256, 256, 0, s>>>(lb.p, (int)((size_t)n * k));
-        k_fill_sentinel<double><<<256, 256, 0, s>>>(ub.p, (int)((size_t)n * k));
+        k_fill_sentinel<double><<<256, 256, 0, s>>>(lb.p, (long)n * k);
+        k_fill_sentinel<double><<<256, 256, 0, s>>>(ub.p, (long)n * k);
         if (!ticket.p) ticket.alloc(1);
         check_launch();
     }
     void rearm(cudaStream_t s)
     {
         if (!lb.p) return;
-        k_fill_sentinel<double><<<256, 256, 0, s>>>(lb.p, (int)((size_t)n * k));
-        k_fill_sentinel<double><<<256, 256, 0, s>>>(ub.p, (int)((size_t)n * k));
+        k_fill_sentinel<double><<<256, 256, 0, s>>>(lb.p, (long)n * k);
+        k_fill_sentinel<double><<<256, 256, 0, s>>>(ub.p, (long)n * k);
         line_xchg_rearm(lx, s);
         line_xchg_rearm(ux, s);
         check_launch();

@@ -105,8 +105,8 @@ struct PrecondDev {
     // re-arm the sentinel buffers (after an aborted solve)
     void rearm(cudaStream_t s)
     {
-        if (lbuf64.n) { k_fill_sentinel<double><<<256, 256, 0, s>>>(lbuf64, n); k_fill_sentinel<double><<<256, 256, 0, s>>>(ubuf64, n); }
-        if (lbuf32.n) { k_fill_sentinel<float><<<256, 256, 0, s>>>(lbuf32, n); k_fill_sentinel<float><<<256, 256, 0, s>>>(ubuf32, n); }
+        if (lbuf64.n) { k_fill_sentinel<double><<<256, 256, 0, s>>>(lbuf64, (long)lbuf64.n); k_fill_sentinel<double><<<256, 256, 0, s>>>(ubuf64, (long)ubuf64.n); }
+        if (lbuf32.n) { k_fill_sentinel<float><<<256, 256, 0, s>>>(lbuf32, (long)lbuf32.n); k_fill_sentinel<float><<<256, 256, 0, s>>>(ubuf32, (long)ubuf32.n); }
         line_xchg_rearm(lx64, s);
         line_xchg_rearm(ux64, s);
         line_xchg_rearm(lx32, s);

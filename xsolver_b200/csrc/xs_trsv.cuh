@@ -403,9 +403,9 @@ __global__ void __launch_bounds__(CH_THREADS) k_trsv_chunked(ChunkArgs<FT> P, co
 
 // Re-arm a solve buffer (used at setup and after an aborted solve).
 template <typename VT>
-__global__ void k_fill_sentinel(VT *b, int n)
+__global__ void k_fill_sentinel(VT *b, long n)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b[i] = Sentinel<VT>::value();
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) b[i] = Sentinel<VT>::value();
 }
 
 }  // namespace xs

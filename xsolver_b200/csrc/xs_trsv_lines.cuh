@@ -928,14 +928,14 @@ inline void line_xchg_ensure(LineXchg<VT> &X, const LineGeo &g, int k, cudaStrea
     X.x.alloc(2 * half);
     X.ctl.alloc(2);
     X.half = half;
-    k_fill_sentinel<VT><<<256, 256, 0, s>>>(X.x.p, (int)(2 * half));
+    k_fill_sentinel<VT><<<256, 256, 0, s>>>(X.x.p, (long)(2 * half));
     check_launch();
 }
 template <typename VT>
 inline void line_xchg_rearm(LineXchg<VT> &X, cudaStream_t s)
 {
     if (!X.x.p) return;
-    k_fill_sentinel<VT><<<256, 256, 0, s>>>(X.x.p, (int)(2 * X.half));
+    k_fill_sentinel<VT><<<256, 256, 0, s>>>(X.x.p, (long)(2 * X.half));
     XS_CUDA(cudaMemsetAsync(X.ctl.p, 0, sizeof(unsigned), s));
 }
 

@@ -173,6 +173,26 @@ def test_wait_times_out_and_recovers(cuda):
             assert np.array_equal(z, oracle.lusolve(F, x))
 
 
+def test_wait_times_out_with_more_patches_than_ctas(cuda):
+    """The same in the middle of a system whose CTAs take several patches
+    each: every CTA ends with its copies landed and its stage barriers in
+    step, and later solves are right."""
+    from xsolver_b200.api import Plan, XsError
+
+    A = _stencil((200, 210, 16), P7)  # 350 patches
+    x = st.rhs_uniform(A.n, 1)
+    with lines_mode(2):
+        P = Plan(A).factor("ilu0")
+        (ref,) = _lusolve(P, x, cuda)
+        P.debug_break_dependency(A.n // 2, True)
+        with pytest.raises(XsError) as e:
+            _lusolve(P, x, cuda)
+        assert e.value.code == 5  # XS_ERR_TRSV_TIMEOUT
+        P.debug_break_dependency(A.n // 2, False)
+        for z in _lusolve(P, x, cuda, reps=3):
+            assert np.array_equal(z, ref)
+
+
 def test_infinities_and_nans_pass_through(cuda):
     """Infinities and NaNs in the right-hand side spread as in the sequential
     solve; a NaN that is not the marker is published like any value."""

@@ -424,6 +424,24 @@ __device__ __forceinline__ int line_wait(const int *p, int target, int *err, uns
     }
     return v;
 }
+// the same, but ended by its own limit only: twice that of any chain of waits
+// the counter's owner can be in (false: given up, error recorded)
+__device__ __forceinline__ bool line_wait_alone(const int *p, int target, int *err, unsigned ns)
+{
+    unsigned long long t0 = 0;
+    for (long it = 1; ld_acquire_cta(p) < target; it++) {
+        __nanosleep(ns);
+        if ((it & 4095) == 0) {
+            const unsigned long long now = gtimer();
+            if (t0 == 0) t0 = now;
+            else if (now - t0 > 16 * WAIT_LIMIT_NS) {
+                atomicOr(err, DEV_TRSV_TIMEOUT);
+                return false;
+            }
+        }
+    }
+    return true;
+}
 // loads and stores at 32-bit shared addresses, in program order with the barriers
 template <typename T>
 __device__ __forceinline__ T lds(uint32_t a)
@@ -532,7 +550,7 @@ __global__ void __launch_bounds__(line_threads_max(KC, W))
     constexpr int L = line_patch(W), T = L * KC, RS = T | 1;
     extern __shared__ __align__(128) unsigned char line_smem[];
     __shared__ __align__(8) uint64_t full[LINE_NS_MAX];
-    __shared__ int s_item, cdone, drained, hcnt[line_poll_warps(LINE_HALO_MAX, KC)];
+    __shared__ int s_item, s_stop, cdone, drained, hcnt[line_poll_warps(LINE_HALO_MAX, KC)];
     __shared__ unsigned s_half;
     const int D = W > 0 ? W : G.D, NV = PIVOT ? 2 * W : D;
     const int S = A.S, NS = A.NS, RL = A.RL, NP = A.NP;
@@ -556,7 +574,10 @@ __global__ void __launch_bounds__(line_threads_max(KC, W))
     }
     pdl_wait();
     if (A.done_flag && *A.done_flag) return;
-    if (tid == 0) s_half = *(volatile unsigned *)(A.ctl + 1);
+    if (tid == 0) {
+        s_half = *(volatile unsigned *)(A.ctl + 1);
+        s_stop = 0;
+    }
     unsigned cnt0 = 0;  // stages consumed by earlier patches of this CTA
     while (true) {
         __syncthreads();  // the previous patch is finished
@@ -575,6 +596,7 @@ __global__ void __launch_bounds__(line_threads_max(KC, W))
         __syncthreads();
         const int item = s_item;
         if (item >= items) break;
+        if (s_stop) continue;  // staging gave up: only the tickets are drawn to the end
         const int rank = item / A.ngroups, grp = item % A.ngroups;
         const int pY = A.patch[2 * rank], pZ = A.patch[2 * rank + 1];
         for (int l = tid; l < L; l += blockDim.x) {
@@ -783,11 +805,23 @@ __global__ void __launch_bounds__(line_threads_max(KC, W))
                     }
                     cp_async_mbar_arrive(&full[slot]);
                 };
-                for (int g = 0; g < NS && g < nst; g++) stage(g);
-                for (int g = NS; g < nst; g++) {
-                    line_wait(&cdone, (g - NS + 1) * S, A.err, 100);
+                // This wait does not end with an error of another one: the
+                // compute threads go on to the last step with every wait of
+                // theirs bounded, and take each stage that is brought, so
+                // the barriers' phases stay in step with them.
+                int g = 0;
+                for (; g < NS && g < nst; g++) stage(g);
+                for (; g < nst; g++) {
+                    if (!line_wait_alone(&cdone, (g - NS + 1) * S, A.err, 100)) break;
                     stage(g);
                 }
+                if (g < nst) s_stop = 1;
+                // no copy is in flight when the patch ends, whatever happened
+                if (h == 0)
+                    for (int q = max(0, g - NS); q < g; q++) {
+                        const unsigned st = cnt0 + (unsigned)q;
+                        if (!mbar_wait_bounded(&full[st % (unsigned)NS], (st / (unsigned)NS) & 1u, A.err)) s_stop = 1;
+                    }
             } else {
                 // re-arm this patch's part of the other half for the next launch
                 VT *xr = A.xb + (s_half ? 0 : A.xb_half) + (long)item * G.nsteps * G.E * KC;

@@ -261,12 +261,19 @@ static __global__ void k_clu_entries(int n, const int *__restrict__ prp, const i
     }
 }
 
-// the largest cluster this kernel can run as (16, else 8, else 0: none),
-// with its shared memory enabled
+// the largest cluster this kernel can run as on the current device (16, else
+// 8, else 0: none), with its shared memory enabled there.  Function
+// attributes belong to one device, so the answer is kept for each.
 template <typename VT, typename FT, typename DT>
 inline int clu_size()
 {
-    static const int c = [] {
+    static std::mutex mu;
+    static signed char known[64] = {};  // by device: 0 not asked yet, else the size + 1
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    std::lock_guard<std::mutex> lock(mu);
+    if (known[dev]) return known[dev] - 1;
+    const int c = [] {
         auto kern = k_lu_cluster<VT, FT, DT>;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLU_SMEM_MAX) != cudaSuccess ||
             cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
@@ -290,6 +297,7 @@ inline int clu_size()
         }
         return 0;
     }();
+    known[dev] = (signed char)(c + 1);
     return c;
 }
 

@@ -477,7 +477,8 @@ int xs_set_trsv_lines(int mode, int min_rows);
 /* Exact LU solves of patterns without a grid schedule on one thread-block
  * cluster, the solution vector in its distributed shared memory (FP64 up to
  * about 450,000 rows): 1 (default), or 0 for the sync-free solve through
- * global memory.  Results are bitwise the same. */
+ * global memory.  Results are bitwise the same.  Takes effect at the next
+ * solve, as xs_set_trsv_block_rows and xs_set_trsv_block_staging do. */
 int xs_set_trsv_cluster(int enable);
 /* Exact LU solves of systems with at most max_rows rows, whose solution
  * vector fits in one SM's shared memory (FP64: 25600 rows), run in one CTA

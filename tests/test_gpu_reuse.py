@@ -205,3 +205,22 @@ def test_preconditioners_in_turn_on_one_handle(cuda):
             assert np.array_equal(a, c), pc
         N.close()
     S.close()
+
+
+def test_switch_of_the_exact_solve_reaches_captured_iterations(cuda):
+    """A handle that has solved (its iterations captured) takes the sync-free
+    solve, two launches, once the cluster solve, one launch, is turned off,
+    and the other way round."""
+    A = mesh(9000, 300, 3, 1)
+    b = st.rhs_uniform(A.n, 3)
+    S = _fresh(A)
+    x, one = S.solve(b), S.launches()
+    with tuning(one_cta=0):
+        y, two = S.solve(b), S.launches()
+        N = _fresh(A)
+        assert np.array_equal(N.solve(b), x) and two == N.launches() > one
+        N.close()
+    assert np.array_equal(x, y)
+    S.solve(b)
+    assert S.launches() == one
+    S.close()

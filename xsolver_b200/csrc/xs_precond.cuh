@@ -126,6 +126,9 @@ struct PrecondDev {
                               (const void *)lx64.x.p, (const void *)ux64.x.p, (const void *)lx32.x.p,
                               (const void *)ux32.x.p, (const void *)y64.p, (const void *)y32.p})
             key.push_back(q);
+        // the switches that choose an exact solve's kernel at its launch
+        const TrsvTuning &t = trsv_tuning();
+        key.push_back((const void *)((long)t.block_max_rows * 4 + t.lu_staged * 2 + t.cluster));
     }
 
     template <typename VT>

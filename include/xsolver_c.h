@@ -341,6 +341,12 @@ int xs_plan_get_stream(xs_plan_t p, void **stream);
 int xs_plan_debug_break_dependency(xs_plan_t p, int position, int enable);
 /* number of dependency levels of L and U */
 int xs_plan_levels(xs_plan_t p, int *levelsL, int *levelsU);
+/* What the plan's exact solves run on.  info[4] = {schedule of L, of U (0
+ * level order, 1 boxes, 2 lines, 3 row chunks), an FP64 LU solve (0 each
+ * triangle by its schedule, 1 both in one CTA, 2 both on one cluster), the
+ * kernel of an exact ILU(0) (1 lane groups, 2 row per thread, 3 boxes, 4
+ * lines; 0: another factor)}. */
+int xs_plan_schedule(xs_plan_t p, int *info);
 /* average device time in ms of `reps` repetitions of op (0 CSR SpMV FP64,
  * 1 ELL SpMV FP64, 2 CSR SpMV FP32, 3 L solve, 4 U solve, 5 LU solve,
  * 6 ELL SpMV FP32) on internal buffers, timed with CUDA events on the plan's
@@ -480,6 +486,10 @@ int xs_set_trsv_lines(int mode, int min_rows);
  * global memory.  Results are bitwise the same.  Takes effect at the next
  * solve, as xs_set_trsv_block_rows and xs_set_trsv_block_staging do. */
 int xs_set_trsv_cluster(int enable);
+/* Every option of the exact solves' schedules (xs_set_trsv_*, their
+ * environment variables read again) back to its default.  A box size, once
+ * set, and the lines' row limits have no other way back. */
+int xs_reset_trsv_tuning(void);
 /* Exact LU solves of systems with at most max_rows rows, whose solution
  * vector fits in one SM's shared memory (FP64: 25600 rows), run in one CTA
  * that walks the dependency levels with a block barrier between them

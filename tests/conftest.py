@@ -21,6 +21,18 @@ def gpu_available():
         return False
 
 
+@pytest.fixture(autouse=True)
+def schedule_defaults(request):
+    """The options of the exact solves' schedules are process-wide, and some
+    (a box size, the lines' row limits) have no setter that undoes them:
+    every GPU test ends with all of them at their defaults."""
+    yield
+    if "cuda" in request.fixturenames:
+        from xsolver_b200 import _lib
+
+        assert _lib.lib().xs_reset_trsv_tuning() == 0
+
+
 @pytest.fixture(scope="session")
 def cuda():
     if not gpu_available():

@@ -59,6 +59,7 @@ def test_batched_lusolve_bitwise_per_column(cuda, k, box_layout):
     A = st.varcoef3d_7pt(26, 1)
     with tiles(box_layout):
         P = Plan(A).factor("ilu0")
+    assert P.schedule()["L"] == P.schedule()["U"] == ("boxes" if box_layout else "levels")
     X = np.stack([st.rhs_uniform(A.n, s) for s in range(k)], axis=1)  # (n, k)
     dX = torch.from_numpy(np.ascontiguousarray(X)).to(cuda)
     dZ = torch.zeros_like(dX)

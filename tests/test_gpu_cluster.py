@@ -82,6 +82,7 @@ def test_lusolve_fp64_bitwise_vs_oracle(cuda, n, reach, per_row, dense):
     x = st.rhs_uniform(n, 7)
     with cluster_mode(1):
         P = Plan(A).factor("ilu0")
+        assert P.schedule()["lu"] == ("cluster" if F.lci.size else "halves")  # one row: nothing to hand over
         for z in _lusolve(P, x, cuda, reps=3):
             assert np.array_equal(z, oracle.lusolve(F, x))
 
@@ -96,6 +97,7 @@ def test_reduced_precision_equals_sync_free(cuda, prec):
     for on in (1, 0):
         with cluster_mode(on):
             P = Plan(A).factor("ilu0").set_factor_precision(prec)
+            assert P.schedule()["lu"] == ("cluster" if on else "halves")
             outs += _lusolve(P, x, cuda, reps=2)
     for z in outs[1:]:
         assert np.array_equal(z, outs[0])
@@ -111,6 +113,7 @@ def test_wait_times_out_and_recovers(cuda):
     x = st.rhs_uniform(A.n, 1)
     with cluster_mode(1):
         P = Plan(A).factor("ilu0")
+        assert P.schedule()["lu"] == "cluster"
         P.debug_break_dependency(A.n - 1, True)
         with pytest.raises(XsError) as e:
             _lusolve(P, x, cuda)
@@ -154,7 +157,9 @@ def test_default_choice_bitwise_vs_oracle(cuda, n):
 
     A = mesh(n, 60, 3, n)
     x = st.rhs_uniform(n, 3)
-    for z in _lusolve(Plan(A).factor("ilu0"), x, cuda, reps=2):
+    P = Plan(A).factor("ilu0")
+    assert P.schedule()["L"] == "levels" and P.schedule()["lu"] == ("one_cta" if n < 4096 else "cluster")
+    for z in _lusolve(P, x, cuda, reps=2):
         assert np.array_equal(z, oracle.lusolve(oracle.ilu0(A), x))
 
 
@@ -176,5 +181,8 @@ def test_default_choice_of_small_grids(cuda, shape):
     v = np.where(r == c, 6.5, -np.random.default_rng(1).uniform(0.3, 1.0, r.size))
     A = CSRMatrix(i.size, np.concatenate([[0], np.cumsum(np.bincount(r))]), c, v)
     b = st.rhs_uniform(A.n, 3)
-    for w in _lusolve(Plan(A).factor("ilu0"), b, cuda, reps=2):
+    P = Plan(A).factor("ilu0")
+    s = P.schedule()
+    assert (s["L"], s["U"], s["lu"]) == (("lines", "lines", "halves") if A.n >= 4096 else ("levels", "levels", "one_cta"))
+    for w in _lusolve(P, b, cuda, reps=2):
         assert np.array_equal(w, oracle.lusolve(oracle.ilu0(A), b))

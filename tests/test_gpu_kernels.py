@@ -360,10 +360,14 @@ def test_block_and_syncfree_lusolve_bitwise(cuda):
         x = st.rhs_uniform(A.n, 11)
         outs = []
         for rows, staged in ((1 << 30, 1), (1 << 30, 0), (0, 1)):
+            # level order on one CTA or sync-free: no lines, no cluster solve
+            assert L.xs_set_trsv_lines(0, 0) == 0 and L.xs_set_trsv_cluster(0) == 0
             assert L.xs_set_trsv_block_rows(rows) == 0
             assert L.xs_set_trsv_block_staging(staged) == 0
             try:
                 P = Plan(A).factor("ilu0")
+                assert P.schedule()["L"] == P.schedule()["U"] == "levels"
+                assert P.schedule()["lu"] == ("one_cta" if rows else "halves")
                 # device inputs stay referenced until the plan's stream is synchronised
                 # (the solves run on the plan's own stream, not torch's)
                 dx, dx32 = _dev(x, cuda), _dev(x.astype(np.float32), cuda)
@@ -393,6 +397,8 @@ def test_syncfree_wait_times_out_and_recovers(cuda):
     from xsolver_b200.api import Plan, XsError
 
     _lib.lib().xs_set_trsv_block_rows(0)
+    _lib.lib().xs_set_trsv_cluster(0)
+    _lib.lib().xs_set_trsv_lines(0, 0)
     try:
         _timeout_case(cuda, torch, Plan, XsError)
     finally:
@@ -402,6 +408,7 @@ def test_syncfree_wait_times_out_and_recovers(cuda):
 def _timeout_case(cuda, torch, Plan, XsError):
     A = st.poisson3d_7pt(16)
     P = Plan(A).factor("ilu0")
+    assert P.schedule()["L"] == "levels" and P.schedule()["lu"] == "halves"
     F = oracle.ilu0(A)
     x = st.rhs_uniform(A.n, 1)
     z = torch.zeros(A.n, dtype=torch.float64, device=cuda)

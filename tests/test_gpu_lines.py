@@ -34,6 +34,10 @@ class lines_mode:
         _lib.lib().xs_set_trsv_lines(1, 512)
 
 
+def _on_lines(P):
+    return P.schedule()["L"] == P.schedule()["U"] == "lines" and P.schedule()["lu"] == "halves"
+
+
 def _dev(a, cuda):
     import torch
 
@@ -69,6 +73,7 @@ def test_lusolve_fp64_bitwise_vs_oracle(cuda, shape, offs):
     x = st.rhs_uniform(A.n, 7)
     with lines_mode(2):
         P = Plan(A).factor("ilu0")
+        assert _on_lines(P)
         for z in _lusolve(P, x, cuda, reps=4):  # both halves of the exchange buffer, re-armed
             assert np.array_equal(z, oracle.lusolve(F, x))
         (zt,) = _lusolve(P, x, cuda, t=True)
@@ -83,6 +88,7 @@ def test_parilut_fill_bitwise_vs_oracle(cuda):
     x = st.rhs_uniform(A.n, 5)
     with lines_mode(2):
         P = Plan(A).factor("parilut", sweeps=5, fill=2.0, droptol=1e-4)
+        assert _on_lines(P)
         (z,) = _lusolve(P, x, cuda)
     assert np.array_equal(z, oracle.lusolve(F, x))
 
@@ -101,6 +107,7 @@ def test_reduced_precision_equals_level_ordered(cuda, prec, shape, offs):
         for mode in (2, 0):
             with lines_mode(mode):
                 P = Plan(A).factor("ilu0").set_factor_precision(prec)
+                assert _on_lines(P) == (mode == 2)
                 outs.append(_lusolve(P, x, cuda, reps=2))
     finally:
         _lib.lib().xs_set_trsv_block_rows(1 << 30)
@@ -119,6 +126,7 @@ def test_several_right_hand_sides_equal_single_solves(cuda, k, shape, offs):
     X = np.stack([st.rhs_uniform(A.n, c) for c in range(k)], 1)
     with lines_mode(2):
         P = Plan(A).factor("ilu0")
+        assert _on_lines(P)
         dX = _dev(X, cuda)
         for _ in range(2):
             Z = torch.full_like(dX, float("nan"))
@@ -148,6 +156,7 @@ def test_one_triangle_on_lines_the_other_not(cuda):
             F = oracle.ilu0(B)
             with lines_mode(2):
                 P = Plan(B).factor("ilu0")
+                assert (P.schedule()["L"] == "lines") != (P.schedule()["U"] == "lines")
                 for z in _lusolve(P, x, cuda, reps=3):
                     assert np.array_equal(z, oracle.lusolve(F, x))
     finally:
@@ -164,6 +173,7 @@ def test_wait_times_out_and_recovers(cuda):
     x = st.rhs_uniform(A.n, 1)
     with lines_mode(2):
         P = Plan(A).factor("ilu0")
+        assert _on_lines(P)
         P.debug_break_dependency(A.n - 1, True)
         with pytest.raises(XsError) as e:
             _lusolve(P, x, cuda)
@@ -203,7 +213,9 @@ def test_infinities_and_nans_pass_through(cuda):
     x = st.rhs_uniform(A.n, 2)
     x[1000], x[3000] = np.inf, np.nan
     with lines_mode(2):
-        (z,) = _lusolve(Plan(A).factor("ilu0"), x, cuda)
+        P = Plan(A).factor("ilu0")
+        assert _on_lines(P)
+        (z,) = _lusolve(P, x, cuda)
     assert np.array_equal(z, oracle.lusolve(F, x), equal_nan=True)
 
 
@@ -227,6 +239,7 @@ def test_ilu0_on_lines_bitwise_vs_oracle(cuda, shape):
             M.val[0] = 0.0
         with lines_mode(2):
             P = Plan(M).factor("ilu0")
+            assert P.schedule()["ilu0"] == "lines"
             assert np.array_equal(P.lu_values(), oracle.ilu0_values(M))
             assert np.array_equal(P.factor("ilu0").lu_values(), oracle.ilu0_values(M))  # refactorised
 
@@ -245,6 +258,7 @@ def test_repeated_columns_keep_their_order(cuda):
     x = st.rhs_uniform(A.n, 1)
     with lines_mode(2):
         P = Plan(B).factor("ilu0")
+        assert P.schedule()["L"] != "lines"
         (z,) = _lusolve(P, x, cuda)
         F = P.factors()
     y = np.zeros(A.n)

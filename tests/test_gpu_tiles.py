@@ -66,6 +66,7 @@ def test_tiled_lusolve_fp64_bitwise_vs_oracle(cuda, box):
     with tiles_forced(box):
         for A in (st.poisson3d_7pt(40), st.convdiff3d_27pt(22), st.varcoef3d_7pt(30, 2)):
             P = Plan(A).factor("ilu0")
+            assert P.schedule()["L"] == P.schedule()["U"] == "boxes"
             F = oracle.ilu0(A)
             x = st.rhs_uniform(A.n, 7)
             ref = oracle.lusolve(F, x)
@@ -82,6 +83,7 @@ def test_tiled_parilut_fill_bitwise_vs_oracle(cuda):
     x = st.rhs_uniform(A.n, 5)
     with tiles_forced():
         P = Plan(A).factor("parilut", sweeps=5, fill=2.0, droptol=1e-4)
+        assert P.schedule()["L"] == P.schedule()["U"] == "boxes"
         (z,) = _solve64(P, x, cuda)
     assert np.array_equal(z, oracle.lusolve(F, x))
 
@@ -97,6 +99,7 @@ def test_tiled_equals_level_ordered_reduced_precision(cuda, prec):
     for enable in (1, 0):
         with tiles_forced(enable=enable):
             P = Plan(A).factor("ilu0").set_factor_precision(prec)
+            assert P.schedule()["L"] == ("boxes" if enable else "levels")
             z = torch.zeros(A.n, dtype=torch.float32, device=cuda)
             dx = _dev(x, cuda)
             P.lusolve(dx, z)
@@ -116,6 +119,7 @@ def test_tiled_wait_times_out_and_recovers(cuda):
     x = st.rhs_uniform(A.n, 1)
     with tiles_forced((8, 8, 8)):
         P = Plan(A).factor("ilu0")
+        assert P.schedule()["L"] == "boxes"
         P.debug_break_dependency(A.n - 1, True)
         with pytest.raises(XsError) as e:
             _solve64(P, x, cuda)

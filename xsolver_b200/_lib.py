@@ -93,6 +93,7 @@ def _declare(L):
         "xs_plan_get_stream": [C.c_void_p, C.POINTER(C.c_void_p)],
         "xs_plan_debug_break_dependency": [C.c_void_p, C.c_int, C.c_int],
         "xs_plan_levels": [C.c_void_p, _ip, _ip],
+        "xs_plan_schedule": [C.c_void_p, _ip],
         "xs_plan_time_op": [C.c_void_p, C.c_int, C.c_int, C.c_int, _dp],
         "xs_plan_op_bytes": [C.c_void_p, C.c_int, _dp],
         "xs_device_count": [],
@@ -104,6 +105,7 @@ def _declare(L):
         "xs_tri_lines": [C.c_int, _ip, _ip, C.c_int, *([_ip] * 8)],
         "xs_set_trsv_lines": [C.c_int, C.c_int],
         "xs_set_trsv_cluster": [C.c_int],
+        "xs_reset_trsv_tuning": [],
         "xs_tri_tiles": [C.c_int, _ip, _ip, C.c_int, C.c_int, C.c_int, C.c_int, _ip, _ip, _ip, _ip, _ip, _ip, _ip,
                          _ip, _ip],
         "xs_set_ell_index_bits": [C.c_int],

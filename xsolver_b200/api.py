@@ -373,6 +373,15 @@ class Plan:
         check(self._L.xs_plan_levels(self.p, C.byref(a), C.byref(b)), "levels")
         return a.value, b.value
 
+    def schedule(self):
+        """What the exact solves run on: schedules of L and U, how an FP64 LU
+        solve is launched, and the kernel of an exact ILU(0)."""
+        info = np.zeros(4, np.int32)
+        check(self._L.xs_plan_schedule(self.p, _i(info)), "schedule")
+        tri = ("levels", "boxes", "lines", "chunks")
+        return {"L": tri[info[0]], "U": tri[info[1]], "lu": ("halves", "one_cta", "cluster")[info[2]],
+                "ilu0": (None, "groups", "rows", "boxes", "lines")[info[3]]}
+
     def time_op(self, op: str, reps: int = 20, flush_l2: bool = True) -> float:
         ms = C.c_double()
         check(self._L.xs_plan_time_op(self.p, self.OPS[op], reps, 1 if flush_l2 else 0, C.byref(ms)), f"time_op({op})")

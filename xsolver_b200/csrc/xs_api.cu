@@ -117,52 +117,54 @@ static int &ilu_tiles_flag()
     return f;
 }
 
+static TileTuning tile_defaults()
+{
+    TileTuning t;
+    // XS_TRSV_TILES: "0" keeps the level-ordered solve; "tx,ty,tz" sets the box size
+    if (const char *e = getenv("XS_TRSV_TILES")) {
+        int a = 0, b = 0, c = 0;
+        const int k = sscanf(e, "%d,%d,%d", &a, &b, &c);
+        if (k == 1 && a == 0) t.enable = 0;
+        else if (k == 3 && a > 0 && b > 0 && c > 0) { t.enable = 1; t.tx = a; t.ty = b; t.tz = c; t.user_box = 1; }
+    }
+    if (const char *e = getenv("XS_TRSV_TILE_MIN_ROWS")) t.min_rows = std::max(8, atoi(e));
+    if (const char *e = getenv("XS_TRSV_TILE_BLOCKS_PER_SM")) t.blocks_per_sm = std::max(1, atoi(e));
+    return t;
+}
 TileTuning &tile_tuning()
 {
-    static TileTuning t;
-    static bool init = false;
-    if (!init) {
-        // XS_TRSV_TILES: "0" keeps the level-ordered solve; "tx,ty,tz" sets the box size
-        if (const char *e = getenv("XS_TRSV_TILES")) {
-            int a = 0, b = 0, c = 0;
-            const int k = sscanf(e, "%d,%d,%d", &a, &b, &c);
-            if (k == 1 && a == 0) t.enable = 0;
-            else if (k == 3 && a > 0 && b > 0 && c > 0) { t.enable = 1; t.tx = a; t.ty = b; t.tz = c; t.user_box = 1; }
-        }
-        if (const char *e = getenv("XS_TRSV_TILE_MIN_ROWS")) t.min_rows = std::max(8, atoi(e));
-        if (const char *e = getenv("XS_TRSV_TILE_BLOCKS_PER_SM")) t.blocks_per_sm = std::max(1, atoi(e));
-        init = true;
-    }
+    static TileTuning t = tile_defaults();
     return t;
 }
 
+static TrsvTuning trsv_defaults()
+{
+    TrsvTuning t;
+    if (const char *e = getenv("XS_TRSV_BLOCKS_PER_SM")) t.blocks_per_sm = atoi(e);
+    if (const char *e = getenv("XS_TRSV_BACKOFF_NS")) t.backoff_ns = std::max(8, atoi(e));
+    if (const char *e = getenv("XS_TRSV_CHUNK_ROWS")) t.chunk_rows = std::max(0, atoi(e));
+    if (const char *e = getenv("XS_TRSV_BLOCK_ROWS")) t.block_max_rows = std::max(0, atoi(e));
+    if (const char *e = getenv("XS_SWEEP_FUSE")) t.fuse_sweeps = atoi(e) != 0;
+    if (const char *e = getenv("XS_LU_STAGED")) t.lu_staged = atoi(e) != 0;
+    if (const char *e = getenv("XS_SWEEP_BALANCED")) t.balanced_sweep_grid = atoi(e) != 0;
+    if (const char *e = getenv("XS_LU_BATCH")) {  // "rows,entries,buffers"
+        int r = 0, en = 0, b = 0;
+        if (sscanf(e, "%d,%d,%d", &r, &en, &b) == 3 && r >= 32 && en >= 32 && b >= 2 && b <= LUB_MAX_BUFS) {
+            t.lub_rows = r;
+            t.lub_entries = en;
+            t.lub_bufs = b;
+            t.lub_auto = 0;
+        }
+    }
+    if (const char *e = getenv("XS_LU_STAGED_THREADS")) {
+        const int v = atoi(e);
+        t.lu_staged_threads = v >= 32 && v <= LU_BLOCK_THREADS && v % 32 == 0 ? v : 0;
+    }
+    return t;
+}
 TrsvTuning &trsv_tuning()
 {
-    static TrsvTuning t;
-    static bool init = false;
-    if (!init) {
-        if (const char *e = getenv("XS_TRSV_BLOCKS_PER_SM")) t.blocks_per_sm = atoi(e);
-        if (const char *e = getenv("XS_TRSV_BACKOFF_NS")) t.backoff_ns = std::max(8, atoi(e));
-        if (const char *e = getenv("XS_TRSV_CHUNK_ROWS")) t.chunk_rows = std::max(0, atoi(e));
-        if (const char *e = getenv("XS_TRSV_BLOCK_ROWS")) t.block_max_rows = std::max(0, atoi(e));
-        if (const char *e = getenv("XS_SWEEP_FUSE")) t.fuse_sweeps = atoi(e) != 0;
-        if (const char *e = getenv("XS_LU_STAGED")) t.lu_staged = atoi(e) != 0;
-        if (const char *e = getenv("XS_SWEEP_BALANCED")) t.balanced_sweep_grid = atoi(e) != 0;
-        if (const char *e = getenv("XS_LU_BATCH")) {  // "rows,entries,buffers"
-            int r = 0, en = 0, b = 0;
-            if (sscanf(e, "%d,%d,%d", &r, &en, &b) == 3 && r >= 32 && en >= 32 && b >= 2 && b <= LUB_MAX_BUFS) {
-                t.lub_rows = r;
-                t.lub_entries = en;
-                t.lub_bufs = b;
-                t.lub_auto = 0;
-            }
-        }
-        if (const char *e = getenv("XS_LU_STAGED_THREADS")) {
-            const int v = atoi(e);
-            t.lu_staged_threads = v >= 32 && v <= LU_BLOCK_THREADS && v % 32 == 0 ? v : 0;
-        }
-        init = true;
-    }
+    static TrsvTuning t = trsv_defaults();
     return t;
 }
 
@@ -414,6 +416,7 @@ struct Handle {
     DBuf<int> tpos;          // IC(0): position of the transposed entry (-1: none)
     DBuf<double> ic0_tnorm;  // IC(0): droptol * row norms
     int ilu_epoch = 0;
+    int ilu_path = 0;  // kernel of the last exact ILU(0): 1 lane groups, 2 row per thread, 3 boxes, 4 lines
     int max_row_len = -1;  // longest row of the pattern (-1: not yet counted)
     DBuf<unsigned> fticket;
     // box-scheduled exact ILU(0) on the L solve's boxes (k_ilu0_tiles: the
@@ -972,6 +975,7 @@ static void factor_ilu(Handle &h, int kind, int sweeps)
                                    h.ilu_epoch, h.err.p, h.fticket.p};
             k_ilu0_tiles<<<gl, ILU_TILE_THREADS, sm, h.s>>>(args, h.ilu_max_entries, h.ilu_max_lower,
                                                             h.ilu_max_rows);
+            h.ilu_path = 3;
         } else if (on_lines) {
             const LinePlan &P = TL.lines;
             const size_t m = (size_t)P.g.slots();
@@ -992,6 +996,7 @@ static void factor_ilu(Handle &h, int kind, int sweeps)
                                                                       (const double *)nullptr, h.lilu_x, 1, h.lilu_a.p,
                                                                       h.lilu_d.p, (double *)nullptr, nullptr, h.err.p, h.s);
             k_line_ilu_finish<<<g8, 256, 0, h.s>>>(n, h.A.rp.p, h.A.ci.p, h.uptr.p, h.lilu_d.p, h.luv.p);
+            h.ilu_path = 4;
         } else if (ilu_group && G <= 32) {
             const int rpb = 128 / G;
             const int bps = ilu_bps_env ? ilu_bps_env : (G <= 8 ? 4 : 8);
@@ -1004,10 +1009,12 @@ static void factor_ilu(Handle &h, int kind, int sweeps)
             else if (G == 8) go(k_ilu0_groups<8>);
             else if (G == 16) go(k_ilu0_groups<16>);
             else go(k_ilu0_groups<32>);
+            h.ilu_path = 1;
         } else {
             const int gl = std::min((n + 127) / 128, geom().sms * (ilu_bps_env ? ilu_bps_env : 1));
             k_ilu0_rows<<<gl, 128, 0, h.s>>>(n, h.A.rp.p, h.A.ci.p, h.uptr.p, h.M.L.level_perm(), h.luv.p, h.flags.p,
                                              h.ilu_epoch, h.err.p, h.fticket.p, ilu_backoff);
+            h.ilu_path = 2;
         }
         check_launch();
     } else {
@@ -2030,6 +2037,14 @@ int xs_tri_lines(int n, const int *rp, const int *ci, int upper, int *info, int 
         put(rank_of, H.rank_of.data(), H.rank_of.size());
         put(halo, H.halo.data(), H.halo.size());
         put(exp_of, H.exp_of.data(), H.exp_of.size());
+    });
+}
+
+int xs_reset_trsv_tuning(void)
+{
+    return guarded([&] {
+        tile_tuning() = tile_defaults();
+        trsv_tuning() = trsv_defaults();
     });
 }
 

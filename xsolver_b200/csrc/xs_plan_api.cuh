@@ -368,6 +368,19 @@ int xs_plan_levels(xs_plan_t p, int *lL, int *lU)
         if (lU) *lU = h.M.U.nlevels;
     });
 }
+int xs_plan_schedule(xs_plan_t p, int *info)
+{
+    return guarded([&] {
+        if (!p || !info) throw Status(XS_ERR_INVALID);
+        Handle &h = *p->h;
+        if (!h.M.have_factors) throw Status(XS_ERR_ORDER);
+        int slots = 0;
+        info[0] = h.M.L.schedule();
+        info[1] = h.M.U.schedule();
+        info[2] = h.M.exact_path<double, double>(slots);
+        info[3] = p->factor_kind == 0 ? h.ilu_path : 0;
+    });
+}
 int xs_plan_op_bytes(xs_plan_t p, int op, double *bytes)
 {
     return guarded([&] {

@@ -15,6 +15,8 @@ inline bool pc_triangular(int t)
 }
 // ... whose factors have a pattern of their own (threshold factorizations)
 inline bool pc_own_pattern(int t) { return t == PC_PARILUT || t == PC_ILUP || t == PC_ICT; }
+// an exact LU solve: each triangle by its own schedule, both in one CTA, or both on one cluster
+enum ExactPath { EXACT_HALVES = 0, EXACT_ONE_CTA = 1, EXACT_CLUSTER = 2 };
 enum FactorPrec { FP_F64 = 0, FP_F32 = 1, FP_BF16 = 2, FP_F16 = 3 };
 
 template <typename VT>
@@ -174,19 +176,29 @@ struct PrecondDev {
         check_launch();
     }
 
+    // how an exact solve with vectors of VT and factors of FT is launched now
+    // (slots: the cluster solve's)
+    template <typename VT, typename FT>
+    ExactPath exact_path(int &slots) const
+    {
+        slots = lu_cluster_slots<VT, FT, VT>(L, U);
+        if (lu_block_ok<VT>(L, U, slots > 0)) return EXACT_ONE_CTA;
+        return slots ? EXACT_CLUSTER : EXACT_HALVES;
+    }
     template <typename VT, typename FT>
     void apply_exact(const VT *x, VT *z, const int *done_flag, cudaStream_t s)
     {
         if (!L.vals<FT>() || !U.vals<FT>()) throw Status(XS_ERR_ORDER);  // copies not built for this configuration
-        const int slots = lu_cluster_slots<VT, FT, VT>(L, U);
-        if (lu_block_ok<VT>(L, U, slots > 0)) {
+        int slots = 0;
+        const ExactPath path = exact_path<VT, FT>(slots);
+        if (path == EXACT_ONE_CTA) {
             const VT *dinv;
             if constexpr (std::is_same<VT, double>::value) dinv = U.dinv64.p;
             else dinv = U.dinv32.p;
             launch_lu_block<VT, FT, VT>(L, U, dinv, x, z, done_flag, s);
             return;
         }
-        if (slots) {
+        if (path == EXACT_CLUSTER) {
             const VT *dinv;
             if constexpr (std::is_same<VT, double>::value) dinv = U.dinv64.p;
             else dinv = U.dinv32.p;

@@ -935,6 +935,8 @@ struct TriDev {
     bool lined = false;
     LinePlan lines;
     const int *level_perm() const { return tiled || lined ? lvperm.p : perm.p; }
+    // its schedule: 0 level order, 1 boxes, 2 lines, 3 row chunks
+    int schedule() const { return lined ? 2 : tiled ? 1 : chunked ? 3 : 0; }
     // forget the schedule of an earlier pattern (an analysis is built in
     // place): no table stays that the new layout does not write, since the
     // dispatch reads them to see what a triangle has

@@ -504,11 +504,14 @@ int xs_set_trsv_block_rows(int max_rows);
  * 0 loads each row's data from global memory one level ahead.  Same result
  * either way.  Environment XS_LU_STAGED sets it at first use. */
 int xs_set_trsv_block_staging(int enable);
-/* Exact ILU(0) factorisation: 1 on the box schedule of the L solve when L
- * has boxes (entries staged in shared memory, one halo wait per box,
- * barriers between the box's levels), 0 (default; faster as measured) the
- * level-ordered lane groups.  Same factors either way.  Environment
- * XS_ILU_TILES sets it at first use. */
+/* Exact ILU(0) factorisation: 1 on the box schedule of the L solve (entries
+ * staged in shared memory, one halo wait per box, barriers between the box's
+ * levels), for which triangles large enough for boxes (xs_set_trsv_tiles) get
+ * boxes instead of lines (where a box's rows of A do not fit in shared
+ * memory, the lane groups); 0 (default; faster as measured) on the line
+ * schedule of 5- and 7-point patterns, else the level-ordered lane groups.
+ * Same factors either way.  Set before a pattern is analysed, that is before
+ * the first factorisation; environment XS_ILU_TILES sets it at first use. */
 int xs_set_ilu_tiles(int enable);
 /* Jacobi-sweep preconditioner apply: 1 computes sweeps 2 and 3 of each
  * narrow diagonal-slot triangle in one pass (each row recomputes the

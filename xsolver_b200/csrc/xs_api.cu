@@ -104,19 +104,6 @@ bool &vec_fusion_flag()
     return on;
 }
 
-// box-scheduled exact ILU(0) (1) or the level-ordered lane groups (0,
-// default: at 128^3 7-point the box kernel took 10.1 ms against 4.6 ms,
-// each internal level paying global-memory latency for the halo rows' upper
-// parts and the dependency lookups); environment XS_ILU_TILES at first use
-static int &ilu_tiles_flag()
-{
-    static int f = [] {
-        const char *e = getenv("XS_ILU_TILES");
-        return e ? (atoi(e) != 0) : 0;
-    }();
-    return f;
-}
-
 static TileTuning tile_defaults()
 {
     TileTuning t;
@@ -128,6 +115,11 @@ static TileTuning tile_defaults()
         else if (k == 3 && a > 0 && b > 0 && c > 0) { t.enable = 1; t.tx = a; t.ty = b; t.tz = c; t.user_box = 1; }
     }
     if (const char *e = getenv("XS_TRSV_TILE_MIN_ROWS")) t.min_rows = std::max(8, atoi(e));
+    // box-scheduled exact ILU(0) (1) or the line pivots and the level-ordered
+    // lane groups (0, default: at 128^3 7-point the box kernel took 10.1 ms
+    // against 0.4 and 4.6 ms, each internal level paying global-memory
+    // latency for the halo rows' upper parts and the dependency lookups)
+    if (const char *e = getenv("XS_ILU_TILES")) t.ilu_boxes = atoi(e) != 0;
     if (const char *e = getenv("XS_TRSV_TILE_BLOCKS_PER_SM")) t.blocks_per_sm = std::max(1, atoi(e));
     return t;
 }
@@ -954,11 +946,11 @@ static void factor_ilu(Handle &h, int kind, int sweeps)
         const TriDev &TL = h.M.L;
         const bool on_lines = TL.lined && h.M.U.lined && h.nnz == TL.nnz + h.M.U.nnz + n &&  // one diagonal entry a row
                               line_ilu_ok(TL.lines, h.M.U.lines);
-        if (ilu_tiles_flag() && !h.ilu_tiles_built) {
+        if (tile_tuning().ilu_boxes && !h.ilu_tiles_built) {
             build_ilu_tiles(h);
             h.ilu_tiles_built = true;
         }
-        if (h.ilu_tiles && ilu_tiles_flag()) {
+        if (h.ilu_tiles && tile_tuning().ilu_boxes) {
             // box schedule: CTAs per SM as the staged box area allows
             const TriDev &L = h.M.L;
             const size_t sm = std::max<size_t>(h.ilu_tiles_smem, 16);
@@ -1920,7 +1912,7 @@ int xs_set_trsv_block_rows(int max_rows)
 
 int xs_set_ilu_tiles(int enable)
 {
-    return guarded([&] { ilu_tiles_flag() = enable != 0; });
+    return guarded([&] { tile_tuning().ilu_boxes = enable != 0; });
 }
 
 int xs_set_trsv_block_staging(int enable)

@@ -1144,7 +1144,8 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
     // boxes shrink until the rows and halo of one fit in shared memory
     TileHostPlan TP;
     T.clear_schedule();
-    const bool want_lines = !T.chunked && tile_tuning().enable && n >= tile_tuning().line_min_rows &&
+    const bool want_lines = !T.chunked && tile_tuning().enable && !(tile_tuning().ilu_boxes && n >= tile_tuning().min_rows) &&
+                            n >= tile_tuning().line_min_rows &&
                             (tile_tuning().lines == 2 || (tile_tuning().lines && !tile_tuning().user_box));
     const bool want_tiles = !T.chunked && tile_tuning().enable && n >= tile_tuning().min_rows;
     // a row with the same column twice has no place for its second entry on

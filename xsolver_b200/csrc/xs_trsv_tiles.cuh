@@ -89,6 +89,7 @@ struct TileTuning {
     // 12^3 29 / 30, 16^3 41 / 34, 32*32*4 54 / 38, 28^3 164 / 66)
     int line_min_rows = 512;
     int line_min_rows_7pt = 4096;
+    int ilu_boxes = 0;  // ILU(0) on boxes asked for (xs_set_ilu_tiles): qualifying triangles get boxes, not lines
 };
 // Triangles with at least this many entries per row on average start from
 // TILE_DENSE_BOX boxes instead of tx/ty/tz: small boxes, long along x, four

@@ -43,6 +43,18 @@ struct HostIo {
         }
         if (pin) cudaFreeHost(pin);
     }
+    // streams, events and pinned memory, as far as they are not there yet
+    bool create()
+    {
+        for (int t = 0; t < HOSTIO_THREADS; t++) {
+            if (!st[t] && cudaStreamCreateWithFlags(&st[t], cudaStreamNonBlocking) != cudaSuccess) return false;
+            for (cudaEvent_t &e : ev[t])
+                if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return false;
+        }
+        if (cudaMallocHost((void **)&pin, HOSTIO_THREADS * 2 * HOSTIO_CHUNK) == cudaSuccess) return true;
+        pin = nullptr;
+        return false;
+    }
     // whether a copy goes through the stripes: large, and not pinned already
     // (or managed: the driver copies those at full rate by itself)
     bool striped(const void *host, size_t bytes)
@@ -54,17 +66,9 @@ struct HostIo {
             return false;
         }
         if (a.type != cudaMemoryTypeUnregistered) return false;
-        if (!pin) {
-            for (int t = 0; t < HOSTIO_THREADS; t++) {
-                if (!st[t]) XS_CUDA(cudaStreamCreateWithFlags(&st[t], cudaStreamNonBlocking));
-                for (cudaEvent_t &e : ev[t])
-                    if (!e) XS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-            }
-            if (cudaMallocHost((void **)&pin, HOSTIO_THREADS * 2 * HOSTIO_CHUNK) != cudaSuccess) {
-                cudaGetLastError();
-                pin = nullptr;
-                return false;
-            }
+        if (!pin && !create()) {
+            cudaGetLastError();
+            return false;  // the driver's own path needs none of it
         }
         return true;
     }
@@ -126,7 +130,9 @@ struct HostIo {
             return e;
         });
     }
-    // host -> device, ordered after stream s; complete when it returns
+    // host -> device, ordered after stream s.  In stripes it is complete when
+    // it returns; otherwise it is a copy in the order of s, and a pinned
+    // source has to stay as it is until s has been waited for
     void upload(void *dst, const void *src, size_t bytes, cudaStream_t s)
     {
         if (!striped(src, bytes)) {

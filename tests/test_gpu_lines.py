@@ -136,6 +136,27 @@ def test_several_right_hand_sides_equal_single_solves(cuda, k, shape, offs):
                 assert np.array_equal(Z[:, c].cpu().numpy(), oracle.lusolve(F, X[:, c]))
 
 
+@pytest.mark.parametrize("k", [2, 3, 16])
+def test_several_right_hand_sides_of_a_long_reach(cuda, k):
+    """A skewed 7-point pattern whose steps reach back so far that only one
+    column of a line fits in shared memory."""
+    import torch
+    from xsolver_b200.api import Plan
+
+    offs = [(0, 1), (1, -8), (2, 8)]
+    A = _stencil((40, 128), [(0, 0)] + offs + [(-a, -b) for a, b in offs])
+    F = oracle.ilu0(A)
+    X = np.stack([st.rhs_uniform(A.n, c) for c in range(k)], 1)
+    P = Plan(A).factor("ilu0")
+    assert _on_lines(P)
+    dX = _dev(X, cuda)
+    Z = torch.full_like(dX, float("nan"))
+    P.lusolve_batch(dX, Z)
+    P.sync()
+    for c in range(k):
+        assert np.array_equal(Z[:, c].cpu().numpy(), oracle.lusolve(F, X[:, c]))
+
+
 def test_one_triangle_on_lines_the_other_not(cuda):
     """A lower triangle that qualifies beside an upper one that does not: each
     kernel re-arms what the other polls, in either order."""

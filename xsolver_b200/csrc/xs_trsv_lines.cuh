@@ -777,7 +777,7 @@ __global__ void __launch_bounds__(line_threads_max(KC, W))
                 const int tau = tau0 + s, col = grp * KC + c;
                 const int q = t.x + tau;
                 const int row = UPPER ? G.n - 1 - q : q;
-                o = KC == 1 ? (long)row : (long)row * A.k + col;
+                o = (long)row * A.k + col;
                 const bool in = (unsigned)(tau - t.y) < (unsigned)G.nx && (KC == 1 || col < A.k);
                 return in ? t.z + c : -1;  // ring column
             };

@@ -136,6 +136,29 @@ def test_several_right_hand_sides_equal_single_solves(cuda, k, shape, offs):
                 assert np.array_equal(Z[:, c].cpu().numpy(), oracle.lusolve(F, X[:, c]))
 
 
+@pytest.mark.parametrize("shape,offs,ks", [((130, 120, 9), P7, (2, 3, 4, 16)), ((72, 72, 9), P27, (11, 12, 15, 16)),
+                                           ((3200, 130), P5, (14, 15, 16))])
+def test_columns_on_both_sides_of_two_per_line(cuda, shape, offs, ks):
+    """Systems of many patches (135, 90 and 25), with fewer and with more
+    columns than give a line two of them (on 148 SMs 370 patches times columns
+    for 5- and 7-point patterns, 1036 for 27-point ones), odd counts among them."""
+    import torch
+    from xsolver_b200.api import Plan
+
+    A = _stencil(shape, offs)
+    F = oracle.ilu0(A)
+    P = Plan(A).factor("ilu0")
+    assert _on_lines(P)
+    X = np.stack([st.rhs_uniform(A.n, c) for c in range(max(ks))], 1)
+    ref = np.stack([oracle.lusolve(F, X[:, c]) for c in range(max(ks))], 1)
+    for k in ks:
+        dX = _dev(X[:, :k], cuda)
+        Z = torch.full_like(dX, float("nan"))
+        P.lusolve_batch(dX, Z)
+        P.sync()
+        assert np.array_equal(Z.cpu().numpy(), ref[:, :k]), k
+
+
 @pytest.mark.parametrize("k", [2, 3, 16])
 def test_several_right_hand_sides_of_a_long_reach(cuda, k):
     """A skewed 7-point pattern whose steps reach back so far that only one

@@ -514,8 +514,7 @@ inline void launch_trsv_multi(const TriDev &T, int k, unsigned *ticket, const do
         const double *pv = T.pv64.p;
         const int kc = line_kc(T.lines.g, k);
         if (kc == 1) launch_trsv_lines<double, double, double, UPPER, 1>(T.lines, pv, T.lines.mask8.p, dinv, X, k, rhs, out, reset_other, all_done, err, s);
-        else if (kc == 2) launch_trsv_lines<double, double, double, UPPER, 2>(T.lines, pv, T.lines.mask8.p, dinv, X, k, rhs, out, reset_other, all_done, err, s);
-        else launch_trsv_lines<double, double, double, UPPER, 4>(T.lines, pv, T.lines.mask8.p, dinv, X, k, rhs, out, reset_other, all_done, err, s);
+        else launch_trsv_lines<double, double, double, UPPER, 2>(T.lines, pv, T.lines.mask8.p, dinv, X, k, rhs, out, reset_other, all_done, err, s);
     } else if (T.tiled) {
         const int kc = tiles_multi_kc(T, k);
         const int ng = (k + kc - 1) / kc;

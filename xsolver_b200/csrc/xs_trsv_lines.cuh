@@ -38,8 +38,8 @@
 //                     vectors stay in natural order and accesses coalesce
 //
 // Measured on B200, an LU solve in FP64, boxes / lines: 128^3 7-point
-// 932 / 318 us, 80^3 27-point 566 us, 128^2 5-point 90 us (197 us in one
-// CTA), eight right-hand sides at 96^3 415 us.  A 7-point step is about 330
+// 932 / 317 us, 80^3 27-point 2006 / 568 us, 128^2 5-point 87 us (197 us in
+// one CTA), eight right-hand sides at 96^3 919 / 397 us.  A 7-point step is about 330
 // cycles, of which the sums are 40 and storing, a barrier and reading back
 // 67; DRAM stays below 20 % of its rate.
 //
@@ -944,13 +944,20 @@ __global__ void __launch_bounds__(line_threads_max(KC, W))
 }
 
 // ---------------------------------------------------------------- launch
-// columns of one compute line for k right-hand sides: up to 4, fewer when
-// their ring and stages do not fit in shared memory
+// columns of one compute line for k right-hand sides: 1, or 2 when the patches
+// of all columns would take the SMs several times over.  A line of one column
+// has the shorter step; two columns read the factor once.  LU solve with 1 / 2
+// columns per line, us: 7-point 48^3 k = 8 125 / 156; 64^3 k = 8 195 / 212, 12
+// 247 / 234; 96^3 k = 2 240 / 308, 5 307 / 338, 6 339 / 345, 8 430 / 397; 128^3
+// k = 3 389 / 457, 4 454 / 466, 6 599 / 558; 5-point 200^2 k = 16 234 / 316;
+// 27-point 40^3 k = 16 310 / 373, 64^3 k = 12 595 / 633, 16 756 / 669, 80^3
+// k = 8 712 / 790, 10 808 / 796, 16 1248 / 961.  (Four columns fit at 27
+// points only, with stages of one step: 2731 at 80^3 for k = 4.)
 inline int line_kc(const LineGeo &g, int k)
 {
-    for (int kc = k >= 3 ? 4 : k; kc > 1; kc = kc == 4 ? 2 : 1)
-        if (line_cfg(g, g.D, 0, kc, sizeof(double), sizeof(double), sizeof(double), g.mask8() ? 1 : 4, 1).S) return kc;
-    return 1;
+    const long sms = geom().sms, most = g.mask8() ? 5 * sms / 2 : 7 * sms;
+    if (k < 2 || (long)g.npatch * k <= most) return 1;
+    return line_cfg(g, g.D, 0, 2, sizeof(double), sizeof(double), sizeof(double), g.mask8() ? 1 : 4, 1).S ? 2 : 1;
 }
 
 template <typename VT>
@@ -1003,7 +1010,10 @@ inline void launch_trsv_lines(const LinePlan &P, const FT *pv, const uint8_t *ma
         XS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LINE_SMEM_MAX));
         launch_pdl(kern, dim3(grid), dim3(threads), c.smem, s, g, A);
     };
-    // unrolled steps: 2 and 4 measured alike, 8 slower (instruction cache), 1
+    // 13 diagonals (27-point ILU(0)) have an instance of their own: with the
+    // generic one an LU solve takes 921 us at 80^3 instead of 568, 167 at
+    // 16^3 instead of 100.
+    // Unrolled steps: 2 and 4 measured alike, 8 slower (instruction cache), 1
     // slower by a sixth (LU solve 128^3 7-point: 319, 318, 330 and 362 us)
     constexpr int SU = 4;
     const bool unrolled = c.S % SU == 0;

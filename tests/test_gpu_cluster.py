@@ -149,16 +149,19 @@ def test_whole_solve_matches_sync_free(cuda):
     assert np.array_equal(res[0][0], res[1][0]) and np.array_equal(res[0][1], res[1][1])
 
 
-@pytest.mark.parametrize("n", [4095, 4096, 4097, 25600, 25601])
-def test_default_choice_bitwise_vs_oracle(cuda, n):
-    """Around the sizes where the solve in one CTA hands over to the cluster,
-    and where its shared memory ends: the default's result is the oracle's."""
+@pytest.mark.parametrize("n,reach,per_row,path",
+                         [(4095, 4000, 1, "one_cta"), (4096, 60, 3, "one_cta"), (8000, 7900, 2, "cluster"),
+                          (24000, 4000, 6, "cluster"), (25600, 60, 3, "one_cta"), (25601, 60, 3, "cluster")])
+def test_default_choice_bitwise_vs_oracle(cuda, n, reach, per_row, path):
+    """Where the solve in one CTA hands over to the cluster: never below 4096
+    rows, above them where a staged batch holds fewer than three average
+    levels, and where the solution leaves its shared memory."""
     from xsolver_b200.api import Plan
 
-    A = mesh(n, 60, 3, n)
+    A = mesh(n, reach, per_row, n)
     x = st.rhs_uniform(n, 3)
     P = Plan(A).factor("ilu0")
-    assert P.schedule()["L"] == "levels" and P.schedule()["lu"] == ("one_cta" if n < 4096 else "cluster")
+    assert P.schedule()["L"] == "levels" and P.schedule()["lu"] == path
     for z in _lusolve(P, x, cuda, reps=2):
         assert np.array_equal(z, oracle.lusolve(oracle.ilu0(A), x))
 

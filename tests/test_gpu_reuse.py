@@ -60,7 +60,7 @@ class tuning:
 
 def _patterns():
     """(matrix, tuning at its analysis): cluster, lines, boxes, one CTA, sync-free."""
-    M, G, S = mesh(9000, 300, 3, 1), _stencil((24, 25, 26), P7), mesh(300, 20, 2, 2)
+    M, G, S = mesh(26000, 300, 3, 1), _stencil((24, 25, 26), P7), mesh(300, 20, 2, 2)
     B = _stencil((41, 41, 41), P7)
     return {"cluster": (M, {}), "lines": (G, {}), "boxes": (B, dict(lines=0)), "one_cta": (S, {}),
             "sync_free": (M, dict(one_cta=0))}
@@ -211,7 +211,7 @@ def test_switch_of_the_exact_solve_reaches_captured_iterations(cuda):
     """A handle that has solved (its iterations captured) takes the sync-free
     solve, two launches, once the cluster solve, one launch, is turned off,
     and the other way round."""
-    A = mesh(9000, 300, 3, 1)
+    A = mesh(26000, 300, 3, 1)
     b = st.rhs_uniform(A.n, 3)
     S = _fresh(A)
     x, one = S.solve(b), S.launches()

@@ -1711,13 +1711,24 @@ __global__ void __launch_bounds__(LU_BLOCK_THREADS) k_lu_staged(TrsvArgs<FT> L, 
 
 // whether the single-CTA solve serves this pair of plans for vectors of VT
 // (cluster: the cluster solve serves them too.  It hands over between SMs,
-// but loads and sums on 16 of them: LU solve of a mesh, one CTA / cluster, us:
-// 512 rows 51 / 68, 2,184 127 / 125, 8,000 232 / 217, 18,750 381 / 335)
+// but loads and sums on 16 of them.  One CTA stages level batches beside the
+// solution vector, so it is ahead as long as a batch holds several levels,
+// and in FP32 most; the cluster is where the vector leaves too little room
+// for wide levels, or a batch none at all.  LU solve, one CTA / cluster, us,
+// batch rows per level beside them: ParILUT of 16^3 27-point 9 FP64 553 / 786,
+// FP32 314 / 770; 24^3 7-point 8 416 / 453, 298 / 428; random meshes of 9,000
+// and 20,000 rows 9-60 224 / 251, 1760 / 2414; front-numbered meshes of 8,400
+// and 18,954 rows 7-15 237 / 218, 367 / 319, FP32 169 / 208, 274 / 305;
+// 25,230 rows 1.7 625 / 346, FP32 589 / 330; 24,000 rows 0.8 455 / 195;
+// 8,000 rows of 9 levels 2 31 / 21; 37,026 rows FP32, unstaged 432 / 400)
 template <typename VT>
 inline bool lu_block_ok(const TriDev &L, const TriDev &U, bool cluster)
 {
     const TrsvTuning &t = trsv_tuning();
-    if (cluster && t.block_max_rows == 1 << 30 && L.n >= CLU_MIN_ROWS) return false;
+    if (cluster && t.block_max_rows == 1 << 30 && L.n >= CLU_MIN_ROWS) {
+        const int width = L.n / std::max(1, std::max(L.nlevels, U.nlevels));
+        if (!L.nlub || !U.nlub || std::min(L.lub_rows, U.lub_rows) < 3 * width) return false;
+    }
     return !L.chunked && !U.chunked && L.n > 0 && L.n <= t.block_max_rows &&
            (size_t)L.n * sizeof(VT) <= LU_BLOCK_SMEM_MAX && L.lstart.p && U.lstart.p;
 }

@@ -57,11 +57,15 @@ def _lusolve(P, x, cuda, reps=1, t=False):
     return out
 
 
+# patterns with a kernel instance of their own beside 5, 7 and 27 points
+P19 = [o for o in P27 if sum(map(abs, o)) <= 2]
+P13 = P9 + [(0, 2), (0, -2), (2, 0), (-2, 0)]
+
 # one line and one step around a patch (32-128 lines) and a stage (8 steps),
 # several patches in Y and Z, lines shorter and longer than the ring (64)
 SHAPES = [((9, 11, 10), P7), ((17, 33, 9), P7), ((16, 8, 64), P7), ((33, 17, 71), P7), ((40, 41, 42), P7),
           ((12, 13, 14), P27), ((17, 33, 20), P27), ((129, 63), P5), ((128, 128), P5), ((7, 300), P5), ((300, 9), P9),
-          ((11, 12, 13), [o for o in P27 if sum(map(abs, o)) <= 2])]
+          ((11, 12, 13), P19), ((17, 33, 9), P19), ((129, 63), P13), ((9, 300), P13), ((129, 63), P9)]
 
 
 @pytest.mark.parametrize("shape,offs", SHAPES)
@@ -94,7 +98,8 @@ def test_parilut_fill_bitwise_vs_oracle(cuda):
 
 
 @pytest.mark.parametrize("prec", ["fp32", "bf16", "fp16"])
-@pytest.mark.parametrize("shape,offs", [((17, 33, 20), P27), ((33, 17, 71), P7), ((129, 63), P5)])
+@pytest.mark.parametrize("shape,offs", [((17, 33, 20), P27), ((33, 17, 71), P7), ((129, 63), P5),
+                                        ((17, 33, 20), P19), ((129, 63), P9), ((129, 63), P13)])
 def test_reduced_precision_equals_level_ordered(cuda, prec, shape, offs):
     from xsolver_b200 import _lib
     from xsolver_b200.api import Plan
@@ -116,7 +121,8 @@ def test_reduced_precision_equals_level_ordered(cuda, prec, shape, offs):
 
 
 @pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 8, 16])
-@pytest.mark.parametrize("shape,offs", [((33, 17, 30), P7), ((12, 13, 14), P27)])
+@pytest.mark.parametrize("shape,offs", [((33, 17, 30), P7), ((12, 13, 14), P27), ((12, 13, 14), P19), ((33, 40), P9),
+                                        ((33, 40), P13)])
 def test_several_right_hand_sides_equal_single_solves(cuda, k, shape, offs):
     import torch
     from xsolver_b200.api import Plan

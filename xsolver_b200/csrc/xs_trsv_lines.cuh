@@ -953,10 +953,13 @@ __global__ void __launch_bounds__(line_threads_max(KC, W))
 // 27-point 40^3 k = 16 310 / 373, 64^3 k = 12 595 / 633, 16 756 / 669, 80^3
 // k = 8 712 / 790, 10 808 / 796, 16 1248 / 961.  (Four columns fit at 27
 // points only, with stages of one step: 2731 at 80^3 for k = 4.)
+// (4, 6 and 9 diagonals have no two-column instance of their own; with one
+// column 19-point 60^3 k = 16 takes 553 us.)
+constexpr bool line_two_columns(int D) { return D != 4 && D != 6 && D != 9; }
 inline int line_kc(const LineGeo &g, int k)
 {
     const long sms = geom().sms, most = g.mask8() ? 5 * sms / 2 : 7 * sms;
-    if (k < 2 || (long)g.npatch * k <= most) return 1;
+    if (k < 2 || (long)g.npatch * k <= most || !line_two_columns(g.D)) return 1;
     return line_cfg(g, g.D, 0, 2, sizeof(double), sizeof(double), sizeof(double), g.mask8() ? 1 : 4, 1).S ? 2 : 1;
 }
 
@@ -1010,9 +1013,12 @@ inline void launch_trsv_lines(const LinePlan &P, const FT *pv, const uint8_t *ma
         XS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LINE_SMEM_MAX));
         launch_pdl(kern, dim3(grid), dim3(threads), c.smem, s, g, A);
     };
-    // 13 diagonals (27-point ILU(0)) have an instance of their own: with the
-    // generic one an LU solve takes 921 us at 80^3 instead of 568, 167 at
-    // 16^3 instead of 100.
+    // The ILU(0) triangles of 9- and 13-point 2D and 19- and 27-point 3D
+    // patterns (4, 6, 9 and 13 diagonals) have instances of their own, without
+    // which the line schedule is behind one CTA up to about 10,000 rows.  LU
+    // solve in one CTA / generic instance / its own, us: 9-point 100^2 267 /
+    // 300 / 134, 13-point 100^2 293 / 300 / 155, 19-point 12^3 103 / 118 / 61,
+    // 27-point 16^3 179 / 167 / 100; 80^3 - / 921 / 568.
     // Unrolled steps: 2 and 4 measured alike, 8 slower (instruction cache), 1
     // slower by a sixth (LU solve 128^3 7-point: 319, 318, 330 and 362 us)
     constexpr int SU = 4;
@@ -1023,7 +1029,12 @@ inline void launch_trsv_lines(const LinePlan &P, const FT *pv, const uint8_t *ma
     else if (g.D == 2) go(k_trsv_lines<VT, FT, DT, UPPER, KC, 2, PIVOT, 1>);
     else if constexpr (PIVOT) throw Status(XS_ERR_UNSUPPORTED);
     else if (g.D == 13 && c.S % 2 == 0) go(k_trsv_lines<VT, FT, DT, UPPER, KC, 13, false, 2>);
-    else go(k_trsv_lines<VT, FT, DT, UPPER, KC, 0, false, 1>);
+    else if constexpr (KC == 1) {
+        if (g.D == 4 && c.S % 2 == 0) go(k_trsv_lines<VT, FT, DT, UPPER, KC, 4, false, 2>);
+        else if (g.D == 6 && c.S % 2 == 0) go(k_trsv_lines<VT, FT, DT, UPPER, KC, 6, false, 2>);
+        else if (g.D == 9 && c.S % 2 == 0) go(k_trsv_lines<VT, FT, DT, UPPER, KC, 9, false, 2>);
+        else go(k_trsv_lines<VT, FT, DT, UPPER, KC, 0, false, 1>);
+    } else go(k_trsv_lines<VT, FT, DT, UPPER, KC, 0, false, 1>);
 }
 
 // ---------------------------------------------------------------- ILU(0) on the line schedule

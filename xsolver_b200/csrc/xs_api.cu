@@ -838,16 +838,19 @@ static void load_tri_values(Handle &h, TriDev &T, const double *vals, const Fact
     check_launch();
 }
 
-static void load_dinv(Handle &h, const double *vals, const long *diagsrc, bool need32)
+// (in the exact solve's order only where one is configured: c.pos)
+static void load_dinv(Handle &h, const double *vals, const long *diagsrc, bool need32, const FactorCopies &c)
 {
     const int g = geom().sms * 4;
     TriDev &U = h.M.U;
     if (U.dinv64_nat.n != (size_t)h.n) U.dinv64_nat.alloc(h.n);
-    gather_pos_dinv<double>(U, diagsrc, vals, U.dinv64, h.s);
+    if (c.pos) gather_pos_dinv<double>(U, diagsrc, vals, U.dinv64, h.s);
+    else U.dinv64.free();
     k_gather_dinv<double><<<g, 256, 0, h.s>>>(h.n, nullptr, diagsrc, vals, U.dinv64_nat.p);
     if (need32) {
         if (U.dinv32_nat.n != (size_t)h.n) U.dinv32_nat.alloc(h.n);
-        gather_pos_dinv<float>(U, diagsrc, vals, U.dinv32, h.s);
+        if (c.pos) gather_pos_dinv<float>(U, diagsrc, vals, U.dinv32, h.s);
+        else U.dinv32.free();
         k_gather_dinv<float><<<g, 256, 0, h.s>>>(h.n, nullptr, diagsrc, vals, U.dinv32_nat.p);
     }
     check_launch();
@@ -980,7 +983,7 @@ static void factor_ilu(Handle &h, int kind, int sweeps)
             }
             line_xchg_ensure(h.lilu_x, P.g, 1, h.s);
             const int g8 = geom().sms * 8;
-            k_line_pairs<<<g8, 256, 0, h.s>>>(P.g, P.patch.p, h.A.rp.p, h.A.ci.p, h.uptr.p, h.A.v.p, h.lilu_pv.p,
+            k_line_pairs<<<g8, 256, 0, h.s>>>(P.g, P.patch, h.A.rp.p, h.A.ci.p, h.uptr.p, h.A.v.p, h.lilu_pv.p,
                                               h.lilu_mask.p);
             k_line_diag<<<g8, 256, 0, h.s>>>(n, h.uptr.p, h.A.v.p, h.lilu_a.p);
             check_launch();
@@ -1122,9 +1125,11 @@ static void build_precond(Handle &h)
         } else {
             for (TriDev *T : {&M.L, &M.U}) { T->ev64.free(); T->ev32.free(); T->evbf.free(); T->evh.free(); }
         }
-        load_dinv(h, h.fv.p, h.udiag_src.p, need32);
-        M.ensure_buffers64(h.s);
-        if (need32) M.ensure_buffers32(h.s);
+        load_dinv(h, h.fv.p, h.udiag_src.p, need32, fc);
+        if (fc.pos) {  // the exact solves' buffers
+            M.ensure_buffers64(h.s);
+            if (need32) M.ensure_buffers32(h.s);
+        }
         if (h.trsv_mode > 0) M.ensure_sweep_buffers(need32);
         M.have_factors = true;
     } else if (pc_own_pattern(type)) {

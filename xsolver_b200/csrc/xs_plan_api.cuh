@@ -267,7 +267,7 @@ int xs_plan_debug_break_dependency(xs_plan_t p, int position, int enable)
             const LineGeo &g = L.lines.g;
             const int z = position / (g.nx * g.ny), Y = position / g.nx % g.ny + g.c * z;
             std::vector<int> rank((size_t)g.npy * g.npz);
-            XS_CUDA(cudaMemcpy(rank.data(), L.lines.rank_of.p, sizeof(int) * rank.size(), cudaMemcpyDeviceToHost));
+            XS_CUDA(cudaMemcpy(rank.data(), L.lines.rank_of, sizeof(int) * rank.size(), cudaMemcpyDeviceToHost));
             L.lines.brk = enable ? rank[(size_t)(z / g.tz) * g.npy + Y / g.ty] : -1;
             return;
         }

@@ -1033,10 +1033,10 @@ inline void gather_pos_values(const TriDev &T, const double *vals, DBuf<FT> &dst
         const int gl = geom().sms * 8;
         if (P.g.mask8()) {
             auto kern = T.upper ? k_line_vals<true, uint8_t, FT> : k_line_vals<false, uint8_t, FT>;
-            kern<<<gl, 256, 0, s>>>(P.g, P.patch.p, P.mask8.p, T.rp_nat.p, T.src_nat.p, vals, dst.p);
+            kern<<<gl, 256, 0, s>>>(P.g, P.patch, P.mask8.p, T.rp_nat.p, T.src_nat.p, vals, dst.p);
         } else {
             auto kern = T.upper ? k_line_vals<true, uint32_t, FT> : k_line_vals<false, uint32_t, FT>;
-            kern<<<gl, 256, 0, s>>>(P.g, P.patch.p, P.mask32.p, T.rp_nat.p, T.src_nat.p, vals, dst.p);
+            kern<<<gl, 256, 0, s>>>(P.g, P.patch, P.mask32.p, T.rp_nat.p, T.src_nat.p, vals, dst.p);
         }
     } else {
         k_gather_convert<FT><<<g, 256, 0, s>>>(T.nnz, T.src.p, vals, dst.p);
@@ -1048,7 +1048,7 @@ inline void gather_pos_dinv(const TriDev &U, const long *diagsrc, const double *
 {
     const int g = geom().sms * 4;
     if (dst.n != U.pos_rows()) dst.alloc(U.pos_rows(), 4);
-    if (U.lined) k_line_dinv<DT><<<g, 256, 0, s>>>(U.lines.g, U.lines.patch.p, diagsrc, vals, dst.p);
+    if (U.lined) k_line_dinv<DT><<<g, 256, 0, s>>>(U.lines.g, U.lines.patch, diagsrc, vals, dst.p);
     else k_gather_dinv<DT><<<g, 256, 0, s>>>(U.n, U.perm.p, diagsrc, vals, dst.p);
     check_launch();
 }
@@ -1170,27 +1170,18 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
             (H.g.D != 3 || n >= tile_tuning().line_min_rows_7pt) && !repeats()) {
             T.lined = true;
             LinePlan &P = T.lines;
-            P.g = H.g;
-            auto up = [&](DBuf<int> &b, const std::vector<int> &v) {
-                b.alloc(std::max<size_t>(v.size(), 1));
-                if (!v.empty()) b.upload(v.data(), v.size(), s);
-            };
-            up(P.patch, H.patch);
-            up(P.rank_of, H.rank_of);
-            up(P.halo, H.halo);
-            up(P.exp_of, H.exp_of);
+            H.upload(P, s);
             const int gl = geom().sms * 8;
             if (P.g.mask8()) {
                 P.mask8.alloc(P.g.slots());
                 auto kern = upper ? k_line_masks<true, uint8_t> : k_line_masks<false, uint8_t>;
-                kern<<<gl, 256, 0, s>>>(P.g, P.patch.p, T.rp_nat.p, T.ci_nat.p, P.mask8.p);
+                kern<<<gl, 256, 0, s>>>(P.g, P.patch, T.rp_nat.p, T.ci_nat.p, P.mask8.p);
             } else {
                 P.mask32.alloc(P.g.slots());
                 auto kern = upper ? k_line_masks<true, uint32_t> : k_line_masks<false, uint32_t>;
-                kern<<<gl, 256, 0, s>>>(P.g, P.patch.p, T.rp_nat.p, T.ci_nat.p, P.mask32.p);
+                kern<<<gl, 256, 0, s>>>(P.g, P.patch, T.rp_nat.p, T.ci_nat.p, P.mask32.p);
             }
             check_launch();
-            XS_CUDA(cudaStreamSynchronize(s));  // the host tables go out of scope
         } else if (on_grid && want_tiles) {
             auto shrink = [&]() {
                 int &big = tt.tx >= tt.ty && tt.tx >= tt.tz ? tt.tx : (tt.ty >= tt.tz ? tt.ty : tt.tz);

@@ -148,10 +148,11 @@ inline LineCfg line_cfg(const LineGeo &g, int nv, int items, int KC, size_t vb, 
 // device copy of a schedule's tables (in TriDev)
 struct LinePlan {
     LineGeo g;
-    DBuf<int> patch;    // pY, pZ of each patch in ticket order
-    DBuf<int> rank_of;  // ticket rank of patch (pY, pZ), -1: no lines
-    DBuf<int> halo;     // Yl, Zl of each halo line (relative to the patch)
-    DBuf<int> exp_of;   // per line of a patch: index among the exported lines, or -1
+    // in one buffer: pY, pZ of each patch in ticket order; ticket rank of
+    // patch (pY, pZ), -1: no lines; Yl, Zl of each halo line (relative to the
+    // patch); per line of a patch its index among the exported lines, or -1
+    DBuf<int> tab;
+    const int *patch = nullptr, *rank_of = nullptr, *halo = nullptr, *exp_of = nullptr;
     DBuf<uint8_t> mask8;
     DBuf<uint32_t> mask32;
     int brk = -1;       // debugging: rank of a patch made to wait for a value of its own
@@ -160,9 +161,9 @@ struct LinePlan {
 // exchange buffer of one consumer (a preconditioner's own solves, or a batch)
 template <typename VT>
 struct LineXchg {
-    DBuf<VT> x;          // two halves
-    DBuf<unsigned> ctl;  // ticket, current half
+    DBuf<VT> x;  // two halves, and behind them the ticket and the current half
     size_t half = 0;
+    unsigned *ctl() const { return (unsigned *)(x.p + 2 * half); }
 };
 
 // Host half of the plan from a detected grid.  False when the pattern does
@@ -172,6 +173,23 @@ struct LineXchg {
 struct LineHost {
     LineGeo g;
     std::vector<int> patch, rank_of, halo, exp_of;
+    // the tables into the plan's buffer, in the order of its pointers
+    void upload(LinePlan &P, cudaStream_t s) const
+    {
+        std::vector<int> all;
+        const int **at[4] = {&P.patch, &P.rank_of, &P.halo, &P.exp_of};
+        const std::vector<int> *v[4] = {&patch, &rank_of, &halo, &exp_of};
+        size_t off[4];
+        for (int k = 0; k < 4; k++) {
+            off[k] = all.size();
+            all.insert(all.end(), v[k]->begin(), v[k]->end());
+        }
+        P.g = g;
+        P.tab.alloc(std::max<size_t>(all.size(), 1));
+        P.tab.upload(all.data(), all.size(), s);
+        XS_CUDA(cudaStreamSynchronize(s));  // `all` goes out of scope
+        for (int k = 0; k < 4; k++) *at[k] = P.tab.p + off[k];
+    }
 };
 
 inline bool line_layout(int n, long nnz, const TileGrid &G, int sms, LineHost &h)
@@ -969,8 +987,7 @@ inline void line_xchg_ensure(LineXchg<VT> &X, const LineGeo &g, int k, cudaStrea
     const int kc = line_kc(g, k), ng = (k + kc - 1) / kc;
     const size_t half = (size_t)g.npatch * ng * g.nsteps * g.E * kc;
     if (X.half == half && X.x.p) return;
-    X.x.alloc(2 * half);
-    X.ctl.alloc(2);
+    X.x.alloc(2 * half, 2 * sizeof(unsigned) / sizeof(VT) + 1);  // zeroed
     X.half = half;
     k_fill_sentinel<VT><<<256, 256, 0, s>>>(X.x.p, (long)(2 * half));
     check_launch();
@@ -980,7 +997,7 @@ inline void line_xchg_rearm(LineXchg<VT> &X, cudaStream_t s)
 {
     if (!X.x.p) return;
     k_fill_sentinel<VT><<<256, 256, 0, s>>>(X.x.p, (long)(2 * X.half));
-    XS_CUDA(cudaMemsetAsync(X.ctl.p, 0, sizeof(unsigned), s));
+    XS_CUDA(cudaMemsetAsync(X.ctl(), 0, sizeof(unsigned), s));
 }
 
 template <typename VT, typename FT, typename DT, bool UPPER, int KC, bool PIVOT = false>
@@ -995,11 +1012,11 @@ inline void launch_trsv_lines(const LinePlan &P, const FT *pv, const uint8_t *ma
                                m8 ? 1 : 4, sms);
     if (c.S == 0 || !X.x.p || X.half != (size_t)items * g.nsteps * g.E * KC) throw Status(XS_ERR_ORDER);
     LineArgs<VT, FT, DT> A;
-    A.patch = P.patch.p; A.rank_of = P.rank_of.p; A.halo = P.halo.p; A.exp_of = P.exp_of.p;
+    A.patch = P.patch; A.rank_of = P.rank_of; A.halo = P.halo; A.exp_of = P.exp_of;
     A.pv = pv;
     A.mask = m8 ? (const void *)mask8 : (const void *)P.mask32.p;
     A.dinv = dinv;
-    A.xb = X.x.p; A.xb_half = (long)X.half; A.ctl = X.ctl.p;
+    A.xb = X.x.p; A.xb_half = (long)X.half; A.ctl = X.ctl();
     A.S = c.S; A.NS = c.NS; A.RL = c.RL;
     A.NP = line_poll_warps(g.nh, KC);
     A.k = k; A.ngroups = ng;

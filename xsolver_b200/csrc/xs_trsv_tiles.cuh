@@ -149,12 +149,14 @@ struct TileHostPlan {
 // ---------------------------------------------------------------- grid fit
 struct GridCoord {
     long nx, nxy;
+    // (rows are 32-bit, and so are their divisions: half the time of a scan)
     void of(long q, int &x, int &y, int &z) const
     {
-        z = (int)(q / nxy);
-        const long r = q - (long)z * nxy;
-        y = (int)(r / nx);
-        x = (int)(r - (long)y * nx);
+        const uint32_t q32 = (uint32_t)q, p = (uint32_t)nxy, l = (uint32_t)nx;
+        const uint32_t z32 = q32 / p, r = q32 - z32 * p, y32 = r / l;
+        z = (int)z32;
+        y = (int)y32;
+        x = (int)(r - y32 * l);
     }
 };
 
@@ -294,15 +296,18 @@ inline bool tile_detect(int n, const int *rp, const int *ci, bool upper, TileGri
         // rank the candidates on the sampled rows, then check the best ones
         // on every entry
         std::vector<std::pair<int, int>> rank;  // (sampled reach, candidate)
+        std::vector<std::vector<int>> sampled(cands.size());
         for (int q = 0; q < (int)cands.size(); q++) {
             const GridCoord gc{cands[q].nx, cands[q].nxy};
-            const int r = grid_reach(n, rp, ci, logical, gc, R, v, step);
+            const int r = grid_reach(n, rp, ci, logical, gc, R, sampled[q], step);
             if (r <= R) rank.push_back({r, q});
         }
         std::sort(rank.begin(), rank.end());
         for (const auto &rq : rank) {
             const GridCoord gc{cands[rq.second].nx, cands[rq.second].nxy};
-            const int r = grid_reach(n, rp, ci, logical, gc, R, v);
+            int r = rq.first;
+            if (step == 1) v.swap(sampled[rq.second]);  // the sample was every row
+            else r = grid_reach(n, rp, ci, logical, gc, R, v);
             if (r <= R && r < best_reach) {
                 best_reach = r;
                 g = gc;

@@ -110,10 +110,11 @@ __global__ void __launch_bounds__(256, 8) k_vecop(Op op, RedSlot slot)
 // fixed grid); below it one CTA per 256 elements: the launch and the last
 // block's sum over all partials are what a small vector costs (PCG of 2,400
 // rows: r.z 7.3 / 5.5 us, x and r update 7.6 / 6.8 with 1184 / 10 CTAs).
+// one_wave: full size at any n, for a caller whose next launch should not start beside this one.
 template <class Op>
-inline void vecop(const Op &op, RedSlot slot, cudaStream_t s)
+inline void vecop(const Op &op, RedSlot slot, cudaStream_t s, bool one_wave = false)
 {
-    const int g = std::max(1, std::min(geom().red_grid, (op.n + 255) / 256));
+    const int g = one_wave ? geom().red_grid : std::max(1, std::min(geom().red_grid, (op.n + 255) / 256));
     launch_pdl(k_vecop<Op>, dim3(g), dim3(256), 0, s, op, slot);
 }
 

@@ -366,7 +366,15 @@ struct BicgRun {
             spmv<VT, MT>(*c.A, z2, v, EpiDot2<VT>{st, s, M_BICG_ALPHA}, sl, c.s);
             OpBicgX<VT> ox{n, st, x, r, z1, z2, s, v, rhat, (VT)0, (VT)0};
             ox.vec_ok = aligned16({x, r, z1, z2, s, v, rhat});
-            vecop(ox, sl, c.s);
+            // The next launch is a sweep with about as many CTAs as this
+            // update would have.  Launched early beside it (programmatic
+            // launch), in FP64 it is slower for it than it gains, from about
+            // half the SMs on: a solve with sweeps takes, with one CTA per
+            // 256 elements / a full wave, 27-point 39,304 rows 2.36 / 2.00
+            // ms, 64,000 2.78 / 2.40, 91,125 3.19 / 2.95; 27,000 rows 2.08 /
+            // 2.08, 8,000 1.35 / 1.42; FP32 40^3 3.99 / 4.15.  (Without early
+            // launches 64,000 rows take 2.28 / 2.37.)
+            vecop(ox, sl, c.s, fuse && sizeof(VT) == 8 && n > geom().sms / 2 * 256);
         };
         // the whole iteration as one persistent kernel when it serves this
         // configuration (same vector updates fused into the sweep passes)

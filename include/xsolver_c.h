@@ -395,7 +395,8 @@ int xs_tri_tiles(int n, const int *rowptr, const int *colidx, int upper, int tx,
                  int *prp, int *pci, int *tile_pos, int *tile_lvl, int *lvl_ptr, int *halo_ptr, int *halo_row);
 
 /* Line schedule of a strict triangle's exact solve (host-only; see
- * xs_set_trsv_lines).  Step x + al*Y + be*Z (Y = y + c*z, Z = z in the
+ * xs_set_trsv_lines; the patch shape depends on the device's number of SMs,
+ * 148 where there is none).  Step x + al*Y + be*Z (Y = y + c*z, Z = z in the
  * triangle's logical coordinates) is solved for all lines of a patch of
  * ty*tz lines at once.  info[24] = {fits, nx, ny, nz, c, al, be, lines per
  * patch, ty, tz, reach in Y and Z, ring columns per row of lines, ring

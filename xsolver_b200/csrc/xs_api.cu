@@ -117,7 +117,7 @@ static TileTuning tile_defaults()
     if (const char *e = getenv("XS_TRSV_TILE_MIN_ROWS")) t.min_rows = std::max(8, atoi(e));
     // box-scheduled exact ILU(0) (1) or the line pivots and the level-ordered
     // lane groups (0, default: at 128^3 7-point the box kernel took 10.1 ms
-    // against 0.4 and 4.6 ms, each internal level paying global-memory
+    // against 0.67 and 4.6 ms, each internal level paying global-memory
     // latency for the halo rows' upper parts and the dependency lookups)
     if (const char *e = getenv("XS_ILU_TILES")) t.ilu_boxes = atoi(e) != 0;
     if (const char *e = getenv("XS_TRSV_TILE_BLOCKS_PER_SM")) t.blocks_per_sm = std::max(1, atoi(e));

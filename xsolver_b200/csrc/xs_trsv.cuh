@@ -1706,12 +1706,14 @@ __global__ void __launch_bounds__(LU_BLOCK_THREADS) k_lu_staged(TrsvArgs<FT> L, 
 // solution vector, so it is ahead as long as a batch holds several levels,
 // and in FP32 most; the cluster is where the vector leaves too little room
 // for wide levels, or a batch none at all.  LU solve, one CTA / cluster, us,
-// batch rows per level beside them: ParILUT of 16^3 27-point 9 FP64 553 / 786,
-// FP32 314 / 770; 24^3 7-point 8 416 / 453, 298 / 428; random meshes of 9,000
-// and 20,000 rows 9-60 224 / 251, 1760 / 2414; front-numbered meshes of 8,400
-// and 18,954 rows 7-15 237 / 218, 367 / 319, FP32 169 / 208, 274 / 305;
-// 25,230 rows 1.7 625 / 346, FP32 589 / 330; 24,000 rows 0.8 455 / 195;
-// 8,000 rows of 9 levels 2 31 / 21; 37,026 rows FP32, unstaged 432 / 400)
+// after the average levels that a batch holds: ParILUT of 16^3 27-point (16)
+// FP64 553 / 786, FP32 314 / 770; of 24^3 7-point (11) 416 / 453, 298 / 428;
+// random meshes of 9,000 (32) and 20,000 rows (59) 224 / 251, 1760 / 2414;
+// meshes numbered front to back of 8,400 (23) and 18,954 rows (6.5) 237 / 218,
+// 367 / 319, FP32 169 / 208, 274 / 305, of 25,230 rows (1.8) 625 / 346, FP32
+// 589 / 330; random ones of 24,000 rows (0.8) 455 / 195, of 8,000 rows in 9
+// levels (2.9) 31 / 21 and in 13 (3.1) 44 / 31; 37,026 rows in FP32,
+// unstaged, 432 / 400)
 template <typename VT>
 inline bool lu_block_ok(const TriDev &L, const TriDev &U, bool cluster)
 {

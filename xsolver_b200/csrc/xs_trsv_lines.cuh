@@ -39,9 +39,12 @@
 //
 // Measured on B200, an LU solve in FP64, boxes / lines: 128^3 7-point
 // 932 / 317 us, 80^3 27-point 2006 / 568 us, 128^2 5-point 87 us (197 us in
-// one CTA), eight right-hand sides at 96^3 919 / 397 us.  A 7-point step is about 330
-// cycles, of which the sums are 40 and storing, a barrier and reading back
-// 67; DRAM stays below 20 % of its rate.
+// one CTA), eight right-hand sides at 96^3 919 / 397 us.  One patch alone
+// (16*8 lines of 2000, 7-point) takes 392 cycles a step, of which the sums are
+// 40 and storing, a barrier and reading back 67; a row of eight patches takes
+// 6 us more per hand-off, and at 128^3 (22 hand-offs on the way, 128 CTAs) a
+// step of the chain comes to 817 cycles, half of them hand-offs; DRAM stays
+// below 10 % of its rate.
 //
 // Patches are taken by ticket in an order in which dependencies come first,
 // so a CTA only waits on patches that running CTAs hold: no co-residency is
@@ -234,8 +237,9 @@ inline bool line_layout(int n, long nnz, const TileGrid &G, int sms, LineHost &h
     if (g.maxd > 32) return false;
     // patch shape: the cheapest of the power-of-two shapes by a model of the
     // chain (steps and hand-offs), the factor stream and the steps all
-    // patches take on the GPU's SMs (microseconds; the constants are the
-    // measured step and hand-off of the kernel below, to one digit)
+    // patches take on the GPU's SMs (microseconds; the constants are early
+    // estimates that rank the shapes: a 7-point step takes 0.2 us alone, a
+    // hand-off 4 to 6)
     const int Yext = g.ny + c * (g.nz - 1);
     double best = 1e300;
     {
@@ -1064,7 +1068,7 @@ inline void launch_trsv_lines(const LinePlan &P, const FT *pv, const uint8_t *ma
 // the reference's ilu0_simple in its order, so the factors are bitwise the
 // same; the rest of the factor is one elementwise pass (k_line_ilu_finish).
 // The lane-group kernel pays a cross-SM hand-off per dependency level: 4.6 ms
-// at 128^3 7-point.
+// at 128^3 7-point against 0.67 here (pivots 0.40).
 inline bool line_ilu_ok(const LinePlan &L, const LinePlan &U)
 {
     const LineGeo &a = L.g, &b = U.g;

@@ -485,7 +485,9 @@ int xs_set_trsv_lines(int mode, int min_rows);
  * cluster, the solution vector in its distributed shared memory (FP64 up to
  * about 450,000 rows): 1 (default), or 0 for the sync-free solve through
  * global memory.  Results are bitwise the same.  Takes effect at the next
- * solve, as xs_set_trsv_block_rows and xs_set_trsv_block_staging do. */
+ * solve, as xs_set_trsv_block_rows and xs_set_trsv_block_staging do; a
+ * pattern analysed while one CTA served it best has no cluster tables and
+ * falls back to the sync-free solve when that is turned off later. */
 int xs_set_trsv_cluster(int enable);
 /* Every option of the exact solves' schedules (xs_set_trsv_*, their
  * environment variables read again) back to its default.  A box size, once

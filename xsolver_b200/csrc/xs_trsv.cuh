@@ -1088,6 +1088,14 @@ inline void host_both(A a, B b)
     if (eb) std::rethrow_exception(eb);
 }
 
+// whether the cluster solve is the faster one where one CTA could serve too:
+// the staged batches (nlub of them, lub_rows rows at most) hold fewer than
+// three average levels, or there are none (measured: see lu_block_ok)
+inline bool clu_over_one_cta(int n, int nlevels, int nlub, int lub_rows)
+{
+    return n >= CLU_MIN_ROWS && (nlub == 0 || lub_rows < 3 * (n / std::max(1, nlevels)));
+}
+
 // Build the device plan of a strict triangle (natural CSR rp/ci, src_of maps
 // an entry to its index in the value array) in the layout the tuning selects,
 // plus the natural-order copy used by the Jacobi-sweep mode.
@@ -1275,33 +1283,6 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
                                         T.src.p);
         check_launch();
         T.lstart.alloc(P.nlevels + 1, 4); T.lstart.upload(P.lstart.data(), P.nlevels + 1, s);
-        // tables of the cluster solve, for sizes it can serve
-        const int C = n <= CLU_MAX * (int)(CLU_SMEM_MAX / sizeof(float)) ? clu_size<double, double, double>() : 0;
-        if (C > 0 && T.nnz && P.nlevels > 0) {
-            std::vector<int> lslot((size_t)P.nlevels * C), used(C, 0);
-            for (int l = 0; l < P.nlevels; l++) {
-                const int w = P.lstart[l + 1] - P.lstart[l];
-                for (int c = 0; c < C; c++) {
-                    lslot[(size_t)l * C + c] = used[c];
-                    used[c] += clu_part(w, c + 1, C) - clu_part(w, c, C);
-                }
-            }
-            T.clu_slots = *std::max_element(used.begin(), used.end());
-            if (T.clu_slots < 65536) {
-                T.clu_c = C;
-                T.clu_lslot.alloc(lslot.size()); T.clu_lslot.upload(lslot.data(), lslot.size(), s);
-                T.clu_dep.alloc(m);
-                T.clu_last.alloc(n);
-                DBuf<uint32_t> where;
-                DBuf<int> level;
-                where.alloc(n);
-                level.alloc(n);
-                k_clu_rows<<<g, 256, 0, s>>>(n, P.nlevels, C, T.perm.p, T.lstart.p, T.clu_lslot.p, where.p, level.p);
-                k_clu_entries<<<g, 256, 0, s>>>(n, T.prp.p, T.pci.p, where.p, level.p, T.clu_dep.p, T.clu_last.p);
-                check_launch();
-                XS_CUDA(cudaStreamSynchronize(s));  // before the temporaries are freed
-            }
-        }
         for (int l = 0; l < P.nlevels; l++) T.max_level_rows = std::max(T.max_level_rows, P.lstart[l + 1] - P.lstart[l]);
         // level batches of the staged single-CTA solve (systems it serves only)
         if ((size_t)n * sizeof(double) <= LU_BLOCK_SMEM_MAX) {
@@ -1347,6 +1328,35 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
             T.nlub = (int)b.size() - 1;
             T.lub.alloc(b.size());
             T.lub.upload(b.data(), b.size(), s);
+        }
+        // tables of the cluster solve, for sizes it can serve and where one CTA
+        // does not (lu_block_ok, by this triangle alone)
+        const bool one_cta = trsv_tuning().block_max_rows >= n && !clu_over_one_cta(n, T.nlevels, T.nlub, T.lub_rows);
+        const int C = !one_cta && n <= CLU_MAX * (int)(CLU_SMEM_MAX / sizeof(float)) ? clu_size<double, double, double>() : 0;
+        if (C > 0 && T.nnz && P.nlevels > 0) {
+            std::vector<int> lslot((size_t)P.nlevels * C), used(C, 0);
+            for (int l = 0; l < P.nlevels; l++) {
+                const int w = P.lstart[l + 1] - P.lstart[l];
+                for (int c = 0; c < C; c++) {
+                    lslot[(size_t)l * C + c] = used[c];
+                    used[c] += clu_part(w, c + 1, C) - clu_part(w, c, C);
+                }
+            }
+            T.clu_slots = *std::max_element(used.begin(), used.end());
+            if (T.clu_slots < 65536) {
+                T.clu_c = C;
+                T.clu_lslot.alloc(lslot.size()); T.clu_lslot.upload(lslot.data(), lslot.size(), s);
+                T.clu_dep.alloc(m);
+                T.clu_last.alloc(n);
+                DBuf<uint32_t> where;
+                DBuf<int> level;
+                where.alloc(n);
+                level.alloc(n);
+                k_clu_rows<<<g, 256, 0, s>>>(n, P.nlevels, C, T.perm.p, T.lstart.p, T.clu_lslot.p, where.p, level.p);
+                k_clu_entries<<<g, 256, 0, s>>>(n, T.prp.p, T.pci.p, where.p, level.p, T.clu_dep.p, T.clu_last.p);
+                check_launch();
+                XS_CUDA(cudaStreamSynchronize(s));  // before the temporaries are freed
+            }
         }
     } else {
         level_analysis();
@@ -1718,10 +1728,9 @@ template <typename VT>
 inline bool lu_block_ok(const TriDev &L, const TriDev &U, bool cluster)
 {
     const TrsvTuning &t = trsv_tuning();
-    if (cluster && t.block_max_rows == 1 << 30 && L.n >= CLU_MIN_ROWS) {
-        const int width = L.n / std::max(1, std::max(L.nlevels, U.nlevels));
-        if (!L.nlub || !U.nlub || std::min(L.lub_rows, U.lub_rows) < 3 * width) return false;
-    }
+    if (cluster && t.block_max_rows == 1 << 30 &&
+        clu_over_one_cta(L.n, std::max(L.nlevels, U.nlevels), std::min(L.nlub, U.nlub), std::min(L.lub_rows, U.lub_rows)))
+        return false;
     return !L.chunked && !U.chunked && L.n > 0 && L.n <= t.block_max_rows &&
            (size_t)L.n * sizeof(VT) <= LU_BLOCK_SMEM_MAX && L.lstart.p && U.lstart.p;
 }

@@ -224,3 +224,23 @@ def test_switch_of_the_exact_solve_reaches_captured_iterations(cuda):
     S.solve(b)
     assert S.launches() == one
     S.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "bf16"])
+def test_sweeps_and_exact_solves_in_turn_on_one_handle(cuda, prec):
+    """A handle with Jacobi sweeps has none of the exact solves' buffers; they
+    are there once it is set to exact solves, and both work again after that."""
+    A = _stencil((24, 25, 26), P7)
+    b = st.rhs_uniform(A.n, 3)
+
+    def fresh(mode):
+        S = _fresh(A).pc_set_trsv(mode)
+        return S.set_precision("fp64", "fp32", prec).set_inner(1e-2, 100) if prec != "fp64" else S
+
+    S = fresh(3)
+    for mode in (3, 0, 3, 0):
+        S.pc_set_trsv(mode)
+        N = fresh(mode)
+        assert np.array_equal(S.solve(b), N.solve(b)), mode
+        N.close()
+    S.close()

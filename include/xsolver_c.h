@@ -499,8 +499,9 @@ int xs_reset_trsv_tuning(void);
  * (bitwise the same result as the sync-free solve, without its cross-SM
  * hand-off per level).  0 disables it; default: no row limit beyond the
  * shared-memory one, but systems of at least 4096 rows whose levels are wide
- * for the room that the solution leaves go to the cluster solve where it
- * serves them (xs_set_trsv_cluster).  Environment XS_TRSV_BLOCK_ROWS sets it at first use. */
+ * for the room that the solution leaves, or wide enough with four or five
+ * entries a row in FP64, go to the cluster solve where it serves them
+ * (xs_set_trsv_cluster).  Environment XS_TRSV_BLOCK_ROWS sets it at first use. */
 int xs_set_trsv_block_rows(int max_rows);
 /* Single-CTA LU solve form: 1 (default) copies whole dependency levels, in
  * batches of up to 512 rows and 2048 entries, into shared memory with

@@ -151,11 +151,14 @@ def test_whole_solve_matches_sync_free(cuda):
 
 @pytest.mark.parametrize("n,reach,per_row,path",
                          [(4095, 4000, 1, "one_cta"), (4096, 60, 3, "one_cta"), (8000, 7900, 2, "cluster"),
-                          (24000, 4000, 6, "cluster"), (25600, 60, 3, "one_cta"), (25601, 60, 3, "cluster")])
+                          (24000, 4000, 6, "cluster"), (25600, 60, 3, "one_cta"), (25601, 60, 3, "cluster"),
+                          (10000, 300, 3, "one_cta"), (10000, 300, 5, "cluster"), (10000, 300, 7, "one_cta"),
+                          (10000, 60, 5, "one_cta"), (4000, 300, 5, "one_cta")])
 def test_default_choice_bitwise_vs_oracle(cuda, n, reach, per_row, path):
     """Where the solve in one CTA hands over to the cluster: never below 4096
     rows, above them where a staged batch holds fewer than three average
-    levels, and where the solution leaves its shared memory."""
+    levels, where the solution leaves its shared memory, and on wide enough
+    levels of rows with four or five entries."""
     from xsolver_b200.api import Plan
 
     A = mesh(n, reach, per_row, n)

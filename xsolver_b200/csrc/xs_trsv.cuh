@@ -1090,10 +1090,13 @@ inline void host_both(A a, B b)
 
 // whether the cluster solve is the faster one where one CTA could serve too:
 // the staged batches (nlub of them, lub_rows rows at most) hold fewer than
-// three average levels, or there are none (measured: see lu_block_ok)
-inline bool clu_over_one_cta(int n, int nlevels, int nlub, int lub_rows)
+// three average levels, or there are none; or, in FP64, levels are at least
+// 24 rows wide with 3.5 to 5.5 entries a row (measured: see lu_block_ok)
+inline bool clu_over_one_cta(int n, int nlevels, int nlub, int lub_rows, long nnz, bool fp64)
 {
-    return n >= CLU_MIN_ROWS && (nlub == 0 || lub_rows < 3 * (n / std::max(1, nlevels)));
+    const int width = n / std::max(1, nlevels);
+    return n >= CLU_MIN_ROWS && (nlub == 0 || lub_rows < 3 * width ||
+                                 (fp64 && width >= 24 && 2 * nnz >= 7L * n && 2 * nnz <= 11L * n));
 }
 
 // Build the device plan of a strict triangle (natural CSR rp/ci, src_of maps
@@ -1331,7 +1334,7 @@ inline void build_tri_dev(TriDev &T, int n, const RV &rp, const CV &ci, bool upp
         }
         // tables of the cluster solve, for sizes it can serve and where one CTA
         // does not (lu_block_ok, by this triangle alone)
-        const bool one_cta = trsv_tuning().block_max_rows >= n && !clu_over_one_cta(n, T.nlevels, T.nlub, T.lub_rows);
+        const bool one_cta = trsv_tuning().block_max_rows >= n && !clu_over_one_cta(n, T.nlevels, T.nlub, T.lub_rows, T.nnz, true);
         const int C = !one_cta && n <= CLU_MAX * (int)(CLU_SMEM_MAX / sizeof(float)) ? clu_size<double, double, double>() : 0;
         if (C > 0 && T.nnz && P.nlevels > 0) {
             std::vector<int> lslot((size_t)P.nlevels * C), used(C, 0);
@@ -1715,7 +1718,12 @@ __global__ void __launch_bounds__(LU_BLOCK_THREADS) k_lu_staged(TrsvArgs<FT> L, 
 // but loads and sums on 16 of them.  One CTA stages level batches beside the
 // solution vector, so it is ahead as long as a batch holds several levels,
 // and in FP32 most; the cluster is where the vector leaves too little room
-// for wide levels, or a batch none at all.  LU solve, one CTA / cluster, us,
+// for wide levels, or a batch none at all.  In FP64 the cluster is ahead, too,
+// by 0 to 15 %, on levels of some width whose rows have four or five entries:
+// with fewer a level is too short to share out, with more a lane reads its
+// remote entries in two rounds (random meshes of 10,000 rows, levels of 25 to
+// 45 rows, entries a row 2.9 251 / 282, 3.9 368 / 371, 4.9 508 / 480, 5.8 620 /
+// 629; narrow levels, 9 rows, 3.9 1166 / 1584).  LU solve, one CTA / cluster, us,
 // after the average levels that a batch holds: ParILUT of 16^3 27-point (16)
 // FP64 553 / 786, FP32 314 / 770; of 24^3 7-point (11) 416 / 453, 298 / 428;
 // random meshes of 9,000 (32) and 20,000 rows (59) 224 / 251, 1760 / 2414;
@@ -1729,7 +1737,8 @@ inline bool lu_block_ok(const TriDev &L, const TriDev &U, bool cluster)
 {
     const TrsvTuning &t = trsv_tuning();
     if (cluster && t.block_max_rows == 1 << 30 &&
-        clu_over_one_cta(L.n, std::max(L.nlevels, U.nlevels), std::min(L.nlub, U.nlub), std::min(L.lub_rows, U.lub_rows)))
+        clu_over_one_cta(L.n, std::max(L.nlevels, U.nlevels), std::min(L.nlub, U.nlub), std::min(L.lub_rows, U.lub_rows),
+                         (L.nnz + U.nnz) / 2, sizeof(VT) == 8))
         return false;
     return !L.chunked && !U.chunked && L.n > 0 && L.n <= t.block_max_rows &&
            (size_t)L.n * sizeof(VT) <= LU_BLOCK_SMEM_MAX && L.lstart.p && U.lstart.p;
